@@ -618,8 +618,8 @@ def _output_exact(case, fields, strain, stats, flags):
 
 def exact(case, seed):
     fluid, _ = _cells(case)
-    # about 4 ns a cell and step, and half a second a thousand small operations
-    if fluid * case["steps"] > 3e9 or case["n_cases"] * case["steps"] > 8000:
+    # about 6 ms a step of a small lattice, 4 ns a cell and step of a large one
+    if fluid * case["steps"] > 3e9 or case["n_cases"] * case["steps"] > 3000:
         return None
     dev = "cuda" if torch.cuda.is_available() else "cpu"
     if case["mode"] == "driver":
