@@ -57,32 +57,37 @@ enum : int { M_RHO = 0, M_VX, M_VY, M_VZ, M_FX, M_FY, M_FZ, M_S11, M_S12, M_S13,
 
 // ---------------------------------------------------------------------------------------
 // storage: F64 holds f itself; F32/F16/BF16 hold the shifted value (f - w_q), times the
-// per-lattice scale for the 16-bit types
+// per-lattice scale for the 16-bit types.  raw / put: the stored value as the arithmetic type
+// and back (what the collisions work on); load / store: the population f itself
 // ---------------------------------------------------------------------------------------
 template <int DT> struct Storage;
 template <> struct Storage<0> {
     using T = double; using CT = double;
-    __device__ static __forceinline__ CT from(T v, int, CT) { return v; }
+    __device__ static __forceinline__ CT raw(T v) { return v; }
+    __device__ static __forceinline__ T put(CT v) { return v; }
     __device__ static __forceinline__ CT load(const T* p, int64_t i, int, CT) { return p[i]; }
     __device__ static __forceinline__ void store(T* p, int64_t i, int, CT v, CT) { p[i] = v; }
 };
 template <> struct Storage<1> {
     using T = float; using CT = float;
-    __device__ static __forceinline__ CT from(T v, int q, CT) { return weight<float>(q) + v; }
+    __device__ static __forceinline__ CT raw(T v) { return v; }
+    __device__ static __forceinline__ T put(CT v) { return v; }
     __device__ static __forceinline__ CT load(const T* p, int64_t i, int q, CT) { return weight<float>(q) + p[i]; }
     __device__ static __forceinline__ void store(T* p, int64_t i, int q, CT v, CT) { p[i] = v - weight<float>(q); }
 };
 template <> struct Storage<2> {
     using T = __half; using CT = float;
-    __device__ static __forceinline__ CT from(T v, int q, CT isc) { return weight<float>(q) + __half2float(v) * isc; }
-    __device__ static __forceinline__ CT load(const T* p, int64_t i, int q, CT isc) { return from(p[i], q, isc); }
+    __device__ static __forceinline__ CT raw(T v) { return __half2float(v); }
+    __device__ static __forceinline__ T put(CT v) { return __float2half_rn(v); }
+    __device__ static __forceinline__ CT load(const T* p, int64_t i, int q, CT isc) { return weight<float>(q) + raw(p[i]) * isc; }
     // (v - w) sc as one fused v sc - w sc (four distinct w sc per thread)
     __device__ static __forceinline__ void store(T* p, int64_t i, int q, CT v, CT sc) { p[i] = __float2half_rn(fmaf(v, sc, -(weight<float>(q) * sc))); }
 };
 template <> struct Storage<3> {
     using T = __nv_bfloat16; using CT = float;
-    __device__ static __forceinline__ CT from(T v, int q, CT isc) { return weight<float>(q) + __bfloat162float(v) * isc; }
-    __device__ static __forceinline__ CT load(const T* p, int64_t i, int q, CT isc) { return from(p[i], q, isc); }
+    __device__ static __forceinline__ CT raw(T v) { return __bfloat162float(v); }
+    __device__ static __forceinline__ T put(CT v) { return __float2bfloat16_rn(v); }
+    __device__ static __forceinline__ CT load(const T* p, int64_t i, int q, CT isc) { return weight<float>(q) + raw(p[i]) * isc; }
     __device__ static __forceinline__ void store(T* p, int64_t i, int q, CT v, CT sc) { p[i] = __float2bfloat16_rn(fmaf(v, sc, -(weight<float>(q) * sc))); }
 };
 
@@ -508,12 +513,7 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 #ifndef NNLBM_CHUNK_REGS_F32
 #define NNLBM_CHUNK_REGS_F32 80
 #endif
-// the one-cell cumulant runs packed columns (step_cell_cum_packed) with every
-// single-precision storage type; with FP16/BF16 storage it gets NNLBM_CHUNK_REGS_CUM16
-// registers (72: the packed pairs spill at 64, and 128-thread blocks keep 28 warps per SM)
-#ifndef NNLBM_PACK_DT
-#define NNLBM_PACK_DT(dt) ((dt) != 0)
-#endif
+// the one-cell cumulant with FP16/BF16 storage gets NNLBM_CHUNK_REGS_CUM16 registers
 #ifndef NNLBM_CHUNK_REGS_CUM16
 #define NNLBM_CHUNK_REGS_CUM16 72
 #endif
@@ -526,20 +526,6 @@ struct StepRegs {
                                  : COL == COL_CUM         ? NNLBM_CHUNK_REGS_CUM16
                                                           : NNLBM_CHUNK_REGS;
 };
-
-// a 16-bit stored value as float, and a float rounded to the 16-bit storage type
-template <int DT>
-__device__ __forceinline__ float widen16(typename Storage<DT>::T v)
-{
-    if constexpr (DT == 2) return __half2float(v);
-    else return __bfloat162float(v);
-}
-template <int DT>
-__device__ __forceinline__ typename Storage<DT>::T narrow16(float v)
-{
-    if constexpr (DT == 2) return __float2half_rn(v);
-    else return __float2bfloat16_rn(v);
-}
 
 // ---------------------------------------------------------------------------------------
 // one 32-cell chunk of the fused step (solver/lbm3d/core.h:578-800), one warp, one cell per
@@ -574,45 +560,18 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
         const T* pc = (const T*)a.df + c;
         // halfway bounce-back: which neighbours are walls (CH_HW chunks, odd step only)
         const uint32_t hwm = (ODD && (ch.cflags & CH_HW)) ? a.hw[c] : 0u;
-        CT f[27];
-        // PAIR16: 16-bit storage with BGK or MRT (measured +2 % each; the cumulant measured 3 %
-        // slower): the
-        // planes x = -1 and x = 0 scale and shift as packed pairs on the way in and out
-        constexpr bool PAIR16 = DT >= 2 && (COL == COL_BGK || COL == COL_MRT);
-        if constexpr (PAIR16) {
-            if (!ODD || plain) {
-                // slot q at c, or slot opp(q) at c - c_q
-                auto src = [&](int q) { return (const T*)(ODD ? odd_ld(a, q) : a.slot_even[q]) + c; };
-                const f2 isc2(a.inv_scale, a.inv_scale);
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    const f2 v = mad(f2(widen16<DT>(*src(j)), widen16<DT>(*src(9 + j))), isc2,
-                                     f2(weight<float>(j), weight<float>(9 + j)));
-                    f[j] = v.v.x;
-                    f[9 + j] = v.v.y;
-                }
-#pragma unroll
-                for (int q = 18; q < 27; ++q) f[q] = S::from(*src(q), q, a.inv_scale);
-            }
-        }
-        if constexpr (PAIR16) {
-            if (ODD && !plain) {
-#pragma unroll
-                for (int q = 0; q < 27; ++q)
-                    f[q] = S::from(((hwm >> oppq(q)) & 1u) ? pc[q * qs] : pc[oppq(q) * qs + nbr(q, -1)], q, a.inv_scale);
-            }
-        } else if (!ODD) {
+        CT f[27]; // the stored values
+        if (!ODD) {
             // slot q at c
 #pragma unroll
-            for (int q = 0; q < 27; ++q) f[q] = S::from(((const T*)a.slot_even[q])[c], q, a.inv_scale);
+            for (int q = 0; q < 27; ++q) f[q] = S::raw(((const T*)a.slot_even[q])[c]);
         } else if (plain) {
             // slot opp(q) at c - c_q
 #pragma unroll
-            for (int q = 0; q < 27; ++q) f[q] = S::from(((const T*)odd_ld(a, q))[c], q, a.inv_scale);
+            for (int q = 0; q < 27; ++q) f[q] = S::raw(((const T*)odd_ld(a, q))[c]);
         } else {
 #pragma unroll
-            for (int q = 0; q < 27; ++q)
-                f[q] = S::from(((hwm >> oppq(q)) & 1u) ? pc[q * qs] : pc[oppq(q) * qs + nbr(q, -1)], q, a.inv_scale);
+            for (int q = 0; q < 27; ++q) f[q] = S::raw(((hwm >> oppq(q)) & 1u) ? pc[q * qs] : pc[oppq(q) * qs + nbr(q, -1)]);
         }
         CT fx = a.fx, fy = a.fy, fz = a.fz;
         if (a.cy_mode == CY_REF_FD && !(ch.periodic & bit)) {
@@ -624,39 +583,22 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
         // a runtime branch inside it)
         CT Sl[6];
         const CYParams<CT> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
-        step_cell<CT, COL, CT, NNLBM_PACK_DT(DT) ? DT : 0>(f, fx, fy, fz, a.nu, a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, Sl, rho, ux, uy, uz);
+        step_cell<CT, COL, DT, DT != 0, CT>(f, fx, fy, fz, a.nu, a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, a.scale, a.inv_scale,
+                                            Sl, rho, ux, uy, uz);
         // the gather of this step reads the slots written below
         pdl_wait();
         T* ps = (T*)a.df + c;
-        if constexpr (PAIR16) {
-            if (!ODD || plain) {
-                // slot opp(q) at c, or slot q at c + c_q
-                auto dst = [&](int q) { return (T*)(ODD ? a.slot_odd_st[q] : a.slot_even[oppq(q)]) + c; };
-                const f2 sc2(a.scale, a.scale);
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    const f2 v = mad(f2(f[j], f[9 + j]), sc2, f2(-(weight<float>(j) * a.scale), -(weight<float>(9 + j) * a.scale)));
-                    *dst(j) = narrow16<DT>(v.v.x);
-                    *dst(9 + j) = narrow16<DT>(v.v.y);
-                }
-#pragma unroll
-                for (int q = 18; q < 27; ++q) S::store(dst(q), 0, q, f[q], a.scale);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 27; ++q)
-                    S::store(ps, ((hwm >> q) & 1u) ? oppq(q) * qs : q * qs + nbr(q, 1), q, f[q], a.scale);
-            }
-        } else if (!ODD) {
+        if (!ODD) {
             // slot opp(q) at c
 #pragma unroll
-            for (int q = 0; q < 27; ++q) S::store((T*)a.slot_even[oppq(q)], c, q, f[q], a.scale);
+            for (int q = 0; q < 27; ++q) ((T*)a.slot_even[oppq(q)])[c] = S::put(f[q]);
         } else if (plain) {
             // slot q at c + c_q
 #pragma unroll
-            for (int q = 0; q < 27; ++q) S::store((T*)a.slot_odd_st[q], c, q, f[q], a.scale);
+            for (int q = 0; q < 27; ++q) ((T*)a.slot_odd_st[q])[c] = S::put(f[q]);
         } else {
 #pragma unroll
-            for (int q = 0; q < 27; ++q) S::store(ps, ((hwm >> q) & 1u) ? oppq(q) * qs : q * qs + nbr(q, 1), q, f[q], a.scale);
+            for (int q = 0; q < 27; ++q) ps[((hwm >> q) & 1u) ? oppq(q) * qs : q * qs + nbr(q, 1)] = S::put(f[q]);
         }
         if ((flags & F_MACRO) || a.cy_mode == CY_REF_FD) {
             write_macro<CT>(a, c, rho, ux, uy, uz, fx, fy, fz);
@@ -844,18 +786,15 @@ template <int DT, bool ODD>
 __device__ __forceinline__ void pair_load_adjacent(const CaseArgs<float>& a, int c0, int lane, f2* f)
 {
     using T = typename Storage<DT>::T;
-    const f2 isc(a.inv_scale);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
         const void* p = ODD ? odd_ld(a, q) : a.slot_even[q];
-        const f2 raw = load_adjacent<DT, ODD>((const T*)p + c0 + 2 * lane);
-        const f2 w(weight<float>(q));
-        f[q] = DT == 1 ? raw + w : mad(raw, isc, w);
+        f[q] = load_adjacent<DT, ODD>((const T*)p + c0 + 2 * lane);
     }
 }
 
-// the rest of a pair once its populations f (raw stored value + weight, or the rest state
-// where the cell does not collide) are in registers: collision, stores, per-cell outputs.
+// the rest of a pair once its stored values f (0, the rest state, where the cell does not
+// collide) are in registers: collision, stores, per-cell outputs.
 // `adj`: an x-adjacent span (lane l holds cells c0 + 2l and c0 + 2l + 1)
 template <int DT, int COL, bool ODD>
 __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const CaseArgs<float>* ap, const Chunk& ca,
@@ -873,15 +812,14 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
         f2 rho, ux, uy, uz;
         f2 Sl[6];
         const CYParams<float> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
-        step_cell<f2, COL, float>(f, fx, fy, fz, f2(a.nu), a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, Sl, rho, ux, uy, uz);
+        step_cell<f2, COL, DT, false, float>(f, fx, fy, fz, f2(a.nu), a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, f2(a.scale),
+                                             f2(a.inv_scale), Sl, rho, ux, uy, uz);
         // the gather of this step reads the slots written below
         pdl_wait();
-        const f2 sc(a.scale);
 #pragma unroll
         for (int q = 0; q < 27; ++q) {
             T* p = (T*)(ODD ? a.slot_odd_st[q] : a.slot_even[oppq(q)]);
-            const f2 w(weight<float>(q));
-            const f2 v = DT == 1 ? f[q] - w : mad(f[q], sc, -(w * sc));
+            const f2 v = f[q];
             if (adj) {
                 store_adjacent<DT, ODD>(p + cA, v);
             } else {
@@ -918,8 +856,8 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
     }
 }
 
-// a pair's populations straight from HBM: the raw stored value + weight of each cell, or
-// the rest state where the cell does not collide
+// a pair's stored values straight from HBM, or 0 (the rest state) where the cell does not
+// collide
 template <int DT, bool ODD>
 __device__ __forceinline__ void pair_load(const CaseArgs<float>& a, const Chunk& ca, const Chunk& cb, int lane, f2* f)
 {
@@ -927,13 +865,10 @@ __device__ __forceinline__ void pair_load(const CaseArgs<float>& a, const Chunk&
     const unsigned bit = 1u << lane;
     const bool fa = (ca.fluid & bit) != 0, fb = (cb.fluid & bit) != 0;
     const int cA = ca.c0 + lane, cB = cb.c0 + lane;
-    const f2 isc(a.inv_scale);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
         const T* p = (const T*)(ODD ? odd_ld(a, q) : a.slot_even[q]);
-        const f2 raw(pair_get<DT>(p + cA, fa), pair_get<DT>(p + cB, fb));
-        const f2 w(weight<float>(q));
-        f[q] = DT == 1 ? raw + w : mad(raw, isc, w);
+        f[q] = f2(pair_get<DT>(p + cA, fa), pair_get<DT>(p + cB, fb));
     }
 }
 
@@ -1158,14 +1093,13 @@ __device__ __forceinline__ const char* staged_elem(const CaseArgs<float>& a, con
     return chunk_buf + lo * G::group + hi * G::row + (r + hi + j) * G::sz;
 }
 
-// a pair's populations from its staged windows: the raw stored value + weight of each cell,
-// or the rest state where the cell does not collide
+// a pair's stored values from its staged windows, or 0 (the rest state) where the cell does
+// not collide
 template <int DT, bool ODD>
 __device__ __forceinline__ void staged_pair_load(const CaseArgs<float>& a, const Chunk& ca, const Chunk& cb, bool adj, int lane,
                                                  const char* buf, f2* f)
 {
     using G = StageGeom<DT>;
-    const f2 isc(a.inv_scale);
     if (adj) {
         // lane l: cells 2l, 2l + 1 of the 64-cell span, in chunk l / 16.  Both chunks have the
         // same window offsets (they are 32 cells apart); the even step's pairs are aligned
@@ -1174,16 +1108,13 @@ __device__ __forceinline__ void staged_pair_load(const CaseArgs<float>& a, const
 #pragma unroll
         for (int q = 0; q < 27; ++q) {
             const char* e = staged_elem<DT, ODD>(a, cbuf, ca.c0, q, j);
-            f2 raw;
             if constexpr (DT == 1) {
-                raw = ODD ? f2(((const float*)e)[0], ((const float*)e)[1]) : f2(*(const float2*)e);
+                f[q] = ODD ? f2(((const float*)e)[0], ((const float*)e)[1]) : f2(*(const float2*)e);
             } else {
                 const unsigned w = ODD ? ((unsigned)((const unsigned short*)e)[0] | ((unsigned)((const unsigned short*)e)[1] << 16))
                                        : *(const unsigned*)e;
-                raw = Pair2<DT>::of(w);
+                f[q] = Pair2<DT>::of(w);
             }
-            const f2 w(weight<float>(q));
-            f[q] = DT == 1 ? raw + w : mad(raw, isc, w);
         }
     } else {
         const unsigned bit = 1u << lane;
@@ -1200,9 +1131,7 @@ __device__ __forceinline__ void staged_pair_load(const CaseArgs<float>& a, const
                 va = Cook<DT>::of_bits(*(const unsigned short*)ea);
                 vb = Cook<DT>::of_bits(*(const unsigned short*)eb);
             }
-            const f2 raw(fa ? va : 0.f, fb ? vb : 0.f);
-            const f2 w(weight<float>(q));
-            f[q] = DT == 1 ? raw + w : mad(raw, isc, w);
+            f[q] = f2(fa ? va : 0.f, fb ? vb : 0.f);
         }
     }
 }

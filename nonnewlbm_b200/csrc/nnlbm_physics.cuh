@@ -152,651 +152,6 @@ __device__ __forceinline__ void equilibrium(int eq, CT rho, CT ux, CT uy, CT uz,
 }
 
 // ---------------------------------------------------------------------------------------
-// cumulant collision (Geier et al. 2015) with the reference configuration of
-// solver/lbm3d/lbm_col_cum.h:166-282: shear rate omega1 = 1/(3 nu + 1/2), every other rate
-// 1, A = B = 0, no limiter.  With those rates all cumulants of order >= 3 are reset to
-// zero, so only the central moments up to second order are needed from the forward
-// transform; the backward transform rebuilds orders 4..6 from products of second order
-// ones (G2015 Eq 81-84).
-// ---------------------------------------------------------------------------------------
-template <class CT>
-__device__ __forceinline__ void fwd3(CT m, CT z, CT p, CT u, CT& k0, CT& k1, CT& k2)
-{
-    // k0 = (p+m)+z, k1 = (p-m) - u k0, k2 = (p+m) - 2u (p-m) + u^2 k0
-    const CT s = p + m, d = p - m;
-    k0 = s + z;
-    k1 = mad(-u, k0, d);
-    k2 = mad(u * u, k0, mad(-(CT(2) * u), d, s));
-}
-
-// the coefficients of one axis of the backward transform:
-// z = k0 (1-u^2) - 2u k1 - k2, m = k0 (u^2-u)/2 + k1 (u - 1/2) + k2/2,
-// p = k0 (u^2+u)/2 + k1 (u + 1/2) + k2/2
-template <class CT>
-struct Bwd {
-    CT a, b, c, d, e, ntu;
-    __device__ __forceinline__ explicit Bwd(CT u)
-    {
-        const CT uu = u * u;
-        a = CT(1) - uu; b = CT(0.5) * (uu - u); c = u - CT(0.5); d = CT(0.5) * (uu + u); e = u + CT(0.5); ntu = CT(-2) * u;
-    }
-};
-
-template <class CT>
-__device__ __forceinline__ void bwd3(CT k0, CT k1, CT k2, const Bwd<CT>& w, CT& m, CT& z, CT& p)
-{
-    const CT h = CT(0.5) * k2;
-    z = mad(k0, w.a, mad(w.ntu, k1, -k2));
-    m = mad(k0, w.b, mad(k1, w.c, h));
-    p = mad(k0, w.d, mad(k1, w.e, h));
-}
-
-template <class CT>
-struct CYParams;
-template <class CT>
-__device__ __forceinline__ CT cy_nu_from_central(CT Cxx, CT Cyy, CT Czz, CT Cxy, CT Cxz, CT Cyz, CT rho, const CYParams<CT>& p,
-                                                 CT* S);
-
-// the first half of the forward z pass, which needs no velocity: per (x, y) column of
-// populations (m, z, p) at f[9 ix + 3 iy + 0..2], its sum k0 = (p + m) + z, d = p - m and
-// s = p + m, in place
-template <class CT>
-__device__ __forceinline__ void cum_columns(CT* f)
-{
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        const CT m = f[3 * c], z = f[3 * c + 1], p = f[3 * c + 2];
-        const CT sp = p + m, d = p - m;
-        f[3 * c] = sp + z;
-        f[3 * c + 1] = d;
-        f[3 * c + 2] = sp;
-    }
-}
-
-// density and velocity u = (j + F/2) / rho from the columns of cum_columns: rho sums the
-// column sums, j_z their d, j_y and j_x the column sums' differences across y and x
-template <class CT>
-__device__ __forceinline__ void cum_density_velocity(const CT* k, CT fx, CT fy, CT fz, CT& rho, CT& ux, CT& uy, CT& uz)
-{
-    auto k0 = [&](int ix, int iy) { return k[9 * ix + 3 * iy]; };
-    auto d = [&](int ix, int iy) { return k[9 * ix + 3 * iy + 1]; };
-    const CT rx0 = (k0(0, 0) + k0(0, 2)) + k0(0, 1), rx1 = (k0(1, 0) + k0(1, 2)) + k0(1, 1), rx2 = (k0(2, 0) + k0(2, 2)) + k0(2, 1);
-    rho = (rx0 + rx2) + rx1;
-    const CT ir = CT(1) / rho;
-    ux = ((rx2 - rx0) + fx * CT(0.5)) * ir;
-    uy = (((k0(0, 2) - k0(0, 0)) + (k0(2, 2) - k0(2, 0))) + (k0(1, 2) - k0(1, 0)) + fy * CT(0.5)) * ir;
-    uz = ((((d(0, 0) + d(0, 2)) + (d(2, 0) + d(2, 2))) + ((d(0, 1) + d(2, 1)) + (d(1, 0) + d(1, 2)))) + d(1, 1) + fz * CT(0.5)) * ir;
-}
-
-// the relaxation of the cumulant (lbm_col_cum.h:205-235 with omega2 = 1 and no anti-aliasing
-// terms) from the central moments k of total order <= 2: s receives the post-collision
-// cumulants as central moments (orders 3 and 5 zero).  `cy` non-null: the shear viscosity
-// comes from the Carreau-Yasuda law on k's second moments, S receives the strain rate
-template <class CT, class PT = CT>
-__device__ __forceinline__ void cum_relax(const CT (&k)[3][3][3], CT rho, CT nu, const CYParams<PT>* cy, CT* S, CT (&s)[3][3][3])
-{
-    const CT ir = CT(1) / rho;
-    if (cy) nu = cy_nu_from_central(k[2][0][0], k[0][2][0], k[0][0][2], k[1][1][0], k[1][0][1], k[0][1][1], rho, *cy, S);
-    const CT om = CT(1) / (CT(3) * nu + CT(0.5));
-    const CT k000 = k[0][0][0];
-    // relaxation (lbm_col_cum.h:205-235 with omega2 = 1 and no anti-aliasing terms)
-    const CT s110 = (CT(1) - om) * k[1][1][0];
-    const CT s101 = (CT(1) - om) * k[1][0][1];
-    const CT s011 = (CT(1) - om) * k[0][1][1];
-    const CT e33 = (CT(1) - om) * (k[2][0][0] - k[0][2][0]);
-    const CT e34 = (CT(1) - om) * (k[2][0][0] - k[0][0][2]);
-    const CT s200 = CT(1.0 / 3.0) * (e33 + e34 + k000);
-    const CT s020 = CT(1.0 / 3.0) * (CT(-2) * e33 + e34 + k000);
-    const CT s002 = CT(1.0 / 3.0) * (e33 - CT(2) * e34 + k000);
-    // fourth order from products (Eq 81-82); third and fifth order vanish
-    const CT s211 = (s200 * s011 + CT(2) * s101 * s110) * ir;
-    const CT s121 = (s020 * s101 + CT(2) * s110 * s011) * ir;
-    const CT s112 = (s002 * s110 + CT(2) * s011 * s101) * ir;
-    const CT s220 = (s020 * s200 + CT(2) * s110 * s110) * ir;
-    const CT s022 = (s002 * s020 + CT(2) * s011 * s011) * ir;
-    const CT s202 = (s200 * s002 + CT(2) * s101 * s101) * ir;
-    // sixth order (Eq 84 with the odd orders at zero)
-    const CT s222 = (s200 * s022 + s020 * s202 + s002 * s220 + CT(4) * (s011 * s211 + s101 * s121 + s110 * s112)) * ir
-                    - (CT(16) * s110 * s101 * s011 + CT(4) * (s101 * s101 * s020 + s011 * s011 * s200 + s110 * s110 * s002)
-                       + CT(2) * s200 * s020 * s002) * ir * ir;
-
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-            for (int l = 0; l < 3; ++l) s[i][j][l] = CT(0);
-    s[0][0][0] = k000;
-    s[1][0][0] = -k[1][0][0]; s[0][1][0] = -k[0][1][0]; s[0][0][1] = -k[0][0][1];
-    s[1][1][0] = s110; s[1][0][1] = s101; s[0][1][1] = s011;
-    s[2][0][0] = s200; s[0][2][0] = s020; s[0][0][2] = s002;
-    s[2][1][1] = s211; s[1][2][1] = s121; s[1][1][2] = s112;
-    s[2][2][0] = s220; s[0][2][2] = s022; s[2][0][2] = s202;
-    s[2][2][2] = s222;
-}
-
-// `cy` non-null: the shear viscosity comes from the Carreau-Yasuda law evaluated on this
-// cell's own central second moments (k_200 ... k_011 of the forward transform); S receives
-// the strain rate.  `f`: the columns of cum_columns; the post-collision populations replace
-// them
-template <class CT, class PT = CT>
-__device__ __forceinline__ void collide_cum_columns(CT* f, CT rho, CT ux, CT uy, CT uz, CT nu, const CYParams<PT>* cy = nullptr,
-                                                    CT* S = nullptr)
-{
-    // forward: the z pass's second half over the 9 (x,y) columns (fwd3 from k0, d, s)
-    CT a[3][3][3];
-    const CT uzz = uz * uz, m2uz = CT(-2) * uz;
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy) {
-            const CT c0 = f[9 * ix + 3 * iy], d = f[9 * ix + 3 * iy + 1], sp = f[9 * ix + 3 * iy + 2];
-            a[ix][iy][0] = c0;
-            a[ix][iy][1] = mad(-uz, c0, d);
-            a[ix][iy][2] = mad(uzz, c0, mad(m2uz, d, sp));
-        }
-    // y pass
-    CT b[3][3][3];
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-        for (int kz = 0; kz < 3; ++kz)
-            fwd3<CT>(a[ix][0][kz], a[ix][1][kz], a[ix][2][kz], uy, b[ix][0][kz], b[ix][1][kz], b[ix][2][kz]);
-    // x pass, only the moments of total order <= 2 are used below
-    CT k[3][3][3];
-#pragma unroll
-    for (int ky = 0; ky < 3; ++ky)
-#pragma unroll
-        for (int kz = 0; kz < 3; ++kz)
-            if (ky + kz <= 2) fwd3<CT>(b[0][ky][kz], b[1][ky][kz], b[2][ky][kz], ux, k[0][ky][kz], k[1][ky][kz], k[2][ky][kz]);
-
-    CT s[3][3][3];
-    cum_relax<CT, PT>(k, rho, nu, cy, S, s);
-    // backward: x, y, z (G2015 Eq 88-96), each axis's coefficients made just before its pass
-    {
-        const Bwd<CT> wx(ux);
-#pragma unroll
-        for (int ky = 0; ky < 3; ++ky)
-#pragma unroll
-            for (int kz = 0; kz < 3; ++kz)
-                bwd3<CT>(s[0][ky][kz], s[1][ky][kz], s[2][ky][kz], wx, b[0][ky][kz], b[1][ky][kz], b[2][ky][kz]);
-    }
-    {
-        const Bwd<CT> wy(uy);
-#pragma unroll
-        for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-            for (int kz = 0; kz < 3; ++kz)
-                bwd3<CT>(b[ix][0][kz], b[ix][1][kz], b[ix][2][kz], wy, a[ix][0][kz], a[ix][1][kz], a[ix][2][kz]);
-    }
-    {
-        const Bwd<CT> wz(uz);
-#pragma unroll
-        for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-            for (int iy = 0; iy < 3; ++iy)
-                bwd3<CT>(a[ix][iy][0], a[ix][iy][1], a[ix][iy][2], wz, f[9 * ix + 3 * iy], f[9 * ix + 3 * iy + 1],
-                         f[9 * ix + 3 * iy + 2]);
-    }
-}
-
-// The cumulant step of one cell in single precision with the columns of x = -1 and x = 0
-// packed into f2 (the packed FP32 pipe runs both at once): the z and y passes of both
-// transforms treat the 18 populations of those two x planes as 9 pairs, the x passes (which
-// combine the planes) and the relaxation run scalar.  The operations and their order are
-// those of cum_columns / collide_cum_columns, so the results are bitwise the same.
-#ifndef NNLBM_CUM_PACKED
-#define NNLBM_CUM_PACKED 1
-#endif
-__device__ __forceinline__ void step_cell_cum_packed(float* f, float fx, float fy, float fz, float nu, const CYParams<float>* cy,
-                                                     float* S, float& rho, float& ux, float& uy, float& uz)
-{
-    // z pass, first half: per column (iy) of the planes ix = 0, 1 (P) and ix = 2 (Q)
-    f2 c0P[3], dP[3], spP[3];
-    float c0Q[3], dQ[3], spQ[3];
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy) {
-        const f2 m(f[3 * iy], f[9 + 3 * iy]), z(f[3 * iy + 1], f[9 + 3 * iy + 1]), p(f[3 * iy + 2], f[9 + 3 * iy + 2]);
-        spP[iy] = p + m;
-        dP[iy] = p - m;
-        c0P[iy] = spP[iy] + z;
-        const float mq = f[18 + 3 * iy], zq = f[18 + 3 * iy + 1], pq = f[18 + 3 * iy + 2];
-        spQ[iy] = pq + mq;
-        dQ[iy] = pq - mq;
-        c0Q[iy] = spQ[iy] + zq;
-    }
-    {
-        float k[27];
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy) {
-            k[3 * iy] = c0P[iy].v.x; k[9 + 3 * iy] = c0P[iy].v.y; k[18 + 3 * iy] = c0Q[iy];
-            k[3 * iy + 1] = dP[iy].v.x; k[9 + 3 * iy + 1] = dP[iy].v.y; k[18 + 3 * iy + 1] = dQ[iy];
-        }
-        cum_density_velocity<float>(k, fx, fy, fz, rho, ux, uy, uz);
-    }
-    // z pass, second half
-    f2 aP[3][3];
-    float aQ[3][3];
-    {
-        const f2 nuz(-uz), uzz(uz * uz), m2uz(-2.f * uz);
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy) {
-            aP[iy][0] = c0P[iy];
-            aP[iy][1] = mad(nuz, c0P[iy], dP[iy]);
-            aP[iy][2] = mad(uzz, c0P[iy], mad(m2uz, dP[iy], spP[iy]));
-            aQ[iy][0] = c0Q[iy];
-            aQ[iy][1] = mad(-uz, c0Q[iy], dQ[iy]);
-            aQ[iy][2] = mad(uz * uz, c0Q[iy], mad(-2.f * uz, dQ[iy], spQ[iy]));
-        }
-    }
-    // y pass
-    f2 bP[3][3];
-    float bQ[3][3];
-#pragma unroll
-    for (int kz = 0; kz < 3; ++kz) {
-        fwd3<f2>(aP[0][kz], aP[1][kz], aP[2][kz], f2(uy), bP[0][kz], bP[1][kz], bP[2][kz]);
-        fwd3<float>(aQ[0][kz], aQ[1][kz], aQ[2][kz], uy, bQ[0][kz], bQ[1][kz], bQ[2][kz]);
-    }
-    // x pass (scalar), orders <= 2
-    float k[3][3][3];
-#pragma unroll
-    for (int ky = 0; ky < 3; ++ky)
-#pragma unroll
-        for (int kz = 0; kz < 3; ++kz)
-            if (ky + kz <= 2) fwd3<float>(bP[ky][kz].v.x, bP[ky][kz].v.y, bQ[ky][kz], ux, k[0][ky][kz], k[1][ky][kz], k[2][ky][kz]);
-    float s[3][3][3];
-    cum_relax<float, float>(k, rho, nu, cy, S, s);
-    // backward x (scalar): the planes ix = 0, 1 of each (ky, kz) land as one pair
-    {
-        const Bwd<float> wx(ux);
-#pragma unroll
-        for (int ky = 0; ky < 3; ++ky)
-#pragma unroll
-            for (int kz = 0; kz < 3; ++kz) {
-                float m, z, p;
-                bwd3<float>(s[0][ky][kz], s[1][ky][kz], s[2][ky][kz], wx, m, z, p);
-                bP[ky][kz] = f2(m, z);
-                bQ[ky][kz] = p;
-            }
-    }
-    // backward y
-    {
-        const Bwd<f2> wy2{f2(uy)};
-        const Bwd<float> wy(uy);
-#pragma unroll
-        for (int kz = 0; kz < 3; ++kz) {
-            bwd3<f2>(bP[0][kz], bP[1][kz], bP[2][kz], wy2, aP[0][kz], aP[1][kz], aP[2][kz]);
-            bwd3<float>(bQ[0][kz], bQ[1][kz], bQ[2][kz], wy, aQ[0][kz], aQ[1][kz], aQ[2][kz]);
-        }
-    }
-    // backward z, into the populations
-    {
-        const Bwd<f2> wz2{f2(uz)};
-        const Bwd<float> wz(uz);
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy) {
-            f2 m, z, p;
-            bwd3<f2>(aP[iy][0], aP[iy][1], aP[iy][2], wz2, m, z, p);
-            f[3 * iy] = m.v.x; f[9 + 3 * iy] = m.v.y;
-            f[3 * iy + 1] = z.v.x; f[9 + 3 * iy + 1] = z.v.y;
-            f[3 * iy + 2] = p.v.x; f[9 + 3 * iy + 2] = p.v.y;
-            bwd3<float>(aQ[iy][0], aQ[iy][1], aQ[iy][2], wz, f[18 + 3 * iy], f[18 + 3 * iy + 1], f[18 + 3 * iy + 2]);
-        }
-    }
-}
-
-// the cumulant collision from populations f and a given density and velocity
-template <class CT, class PT = CT>
-__device__ __forceinline__ void collide_cum(CT* f, CT rho, CT ux, CT uy, CT uz, CT nu, const CYParams<PT>* cy = nullptr,
-                                            CT* S = nullptr)
-{
-    cum_columns<CT>(f);
-    collide_cum_columns<CT, PT>(f, rho, ux, uy, uz, nu, cy, S);
-}
-
-// ---------------------------------------------------------------------------------------
-// factorised equilibrium of the BGK / KBC schemes (lbm_col_bgk.h:43-53, 85-111):
-// feq_q = -rho X_cx Y_cy Z_cz with Xz = u^2 - 2/3, Xp = -(u^2 + u + 1/3)/2, Xm = Xp + u
-// ---------------------------------------------------------------------------------------
-template <class CT>
-struct FactEq {
-    CT X[3], Y[3], Z[3];
-    __device__ __forceinline__ FactEq(CT ux, CT uy, CT uz)
-    {
-        X[1] = CT(1.0 / 3.0) - CT(1) + ux * ux; X[2] = CT(-0.5) * (X[1] + CT(1) + ux); X[0] = X[2] + ux;
-        Y[1] = CT(1.0 / 3.0) - CT(1) + uy * uy; Y[2] = CT(-0.5) * (Y[1] + CT(1) + uy); Y[0] = Y[2] + uy;
-        Z[1] = CT(1.0 / 3.0) - CT(1) + uz * uz; Z[2] = CT(-0.5) * (Z[1] + CT(1) + uz); Z[0] = Z[2] + uz;
-    }
-    __device__ __forceinline__ CT operator()(int q, CT rho) const { return -rho * X[q / 9] * Y[(q / 3) % 3] * Z[q % 3]; }
-};
-
-// forcing source S_q of lbm_col_bgk.h:57-83
-template <class CT>
-__device__ __forceinline__ CT force_src(int q, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
-{
-    return (CT(3) * ((CT(cxq(q)) - ux) * fx + (CT(cyq(q)) - uy) * fy + (CT(czq(q)) - uz) * fz)) * ir;
-}
-
-// BGK, solver/lbm3d/lbm_col_bgk.h:14-140
-template <class CT>
-__device__ __forceinline__ void collide_bgk(CT* f, CT rho, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz, CT nu)
-{
-    const CT om = CT(1) / (CT(3) * nu + CT(0.5));
-    const CT ir = CT(1) / rho;
-    const FactEq<CT> E(ux, uy, uz);
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const CT feq = E(q, rho);
-        f[q] += (feq - f[q]) * om + (CT(1) - CT(0.5) * om) * force_src<CT>(q, ir, ux, uy, uz, fx, fy, fz) * feq;
-    }
-}
-
-// density and velocity of one cell in single precision from its column sums (the z pass's
-// first half, cum_columns, with the columns of the planes x = -1, 0 as packed pairs), f
-// unchanged
-__device__ __forceinline__ void packed_density_velocity(const float* f, float fx, float fy, float fz, float& rho, float& ux,
-                                                        float& uy, float& uz)
-{
-    float k[27];
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy) {
-        const f2 m(f[3 * iy], f[9 + 3 * iy]), z(f[3 * iy + 1], f[9 + 3 * iy + 1]), p(f[3 * iy + 2], f[9 + 3 * iy + 2]);
-        const f2 d = p - m, c0 = (p + m) + z;
-        const float mq = f[18 + 3 * iy], zq = f[18 + 3 * iy + 1], pq = f[18 + 3 * iy + 2];
-        k[3 * iy] = c0.v.x; k[9 + 3 * iy] = c0.v.y; k[18 + 3 * iy] = (pq + mq) + zq;
-        k[3 * iy + 1] = d.v.x; k[9 + 3 * iy + 1] = d.v.y; k[18 + 3 * iy + 1] = pq - mq;
-    }
-    cum_density_velocity<float>(k, fx, fy, fz, rho, ux, uy, uz);
-}
-
-// BGK of one cell in single precision with the populations of the planes x = -1 and x = 0
-// packed into f2 pairs (the same operations in the same order as collide_bgk; the x = +1
-// plane runs scalar)
-__device__ __forceinline__ void collide_bgk_packed(float* f, float rho, float ux, float uy, float uz, float fx, float fy,
-                                                   float fz, float nu)
-{
-    const float om = 1.f / (3.f * nu + 0.5f);
-    const float ir = 1.f / rho;
-    const float k = 1.f - 0.5f * om;
-    const FactEq<float> E(ux, uy, uz);
-    const f2 rX(-rho * E.X[0], -rho * E.X[1]);
-    const float rX2 = -rho * E.X[2];
-    const f2 A((-1.f - ux) * fx, (0.f - ux) * fx);
-    const float A2 = (1.f - ux) * fx;
-    const f2 om2(om), k2(k), three(3.0), ir2(ir);
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy)
-#pragma unroll
-        for (int iz = 0; iz < 3; ++iz) {
-            const int j = 3 * iy + iz;
-            const float Y = E.Y[iy], Z = E.Z[iz];
-            const float B = ((float)(iy - 1) - uy) * fy, C = ((float)(iz - 1) - uz) * fz;
-            const f2 feq = (rX * f2(Y, Y)) * f2(Z, Z);
-            const f2 src = (three * ((A + f2(B, B)) + f2(C, C))) * ir2;
-            const f2 fv(f[j], f[9 + j]);
-            const f2 nv = fv + mad(feq - fv, om2, (k2 * src) * feq);
-            f[j] = nv.v.x;
-            f[9 + j] = nv.v.y;
-            const float feq1 = (rX2 * Y) * Z;
-            const float src1 = (3.f * ((A2 + B) + C)) * ir;
-            f[18 + j] += (feq1 - f[18 + j]) * om + (k * src1) * feq1;
-        }
-}
-
-// MRT_LES, solver/lbm3d/lbm_col_mrt.h:12-78: second moments relaxed with a Smagorinsky rate,
-// everything rebuilt as w_q [rho (1 + 3 c.u) + 9/2 (c c - I/3) : (P - rho I/3)] form
-// the relaxed second moments of MRT_LES (P, and tr = trace P) from the populations
-template <class CT>
-__device__ __forceinline__ void mrt_moments(const CT* f, CT rho, CT ux, CT uy, CT uz, CT nu, CT& Pxx, CT& Pyy, CT& Pzz, CT& Pxy,
-                                            CT& Pxz, CT& Pyz, CT& tr)
-{
-    Pxx = CT(0); Pyy = CT(0); Pzz = CT(0); Pxy = CT(0); Pxz = CT(0); Pyz = CT(0);
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int cx = cxq(q), cy = cyq(q), cz = czq(q);
-        if (cx) Pxx += f[q];
-        if (cy) Pyy += f[q];
-        if (cz) Pzz += f[q];
-        if (cx * cy > 0) Pxy += f[q]; else if (cx * cy < 0) Pxy -= f[q];
-        if (cx * cz > 0) Pxz += f[q]; else if (cx * cz < 0) Pxz -= f[q];
-        if (cy * cz > 0) Pyz += f[q]; else if (cy * cz < 0) Pyz -= f[q];
-    }
-    const CT Pnxx = Pxx - rho * (CT(1.0 / 3.0) + ux * ux);
-    const CT Pnyy = Pyy - rho * (CT(1.0 / 3.0) + uy * uy);
-    const CT Pnzz = Pzz - rho * (CT(1.0 / 3.0) + uz * uz);
-    const CT Pnxz = Pxz - rho * ux * uz;
-    const CT Pnxy = Pxy - rho * ux * uy;
-    const CT Pnyz = Pyz - rho * uy * uz;
-    const CT Qs = CT(2) * (Pnxx * Pnxx + Pnyy * Pnyy + Pnzz * Pnzz + CT(2) * (Pnxy * Pnxy + Pnxz * Pnxz + Pnyz * Pnyz));
-    const CT tau = CT(3) * nu + CT(0.5);
-    const CT om = CT(2) / (dsqrt<CT>(tau * tau + CT(2) * CT(0.0342) * CT(9) * dsqrt<CT>(Qs) / rho) + tau);
-    Pxx -= om * Pnxx; Pyy -= om * Pnyy; Pzz -= om * Pnzz;
-    Pxy -= om * Pnxy; Pxz -= om * Pnxz; Pyz -= om * Pnyz;
-    tr = Pxx + Pyy + Pzz;
-}
-
-template <class CT>
-__device__ __forceinline__ void collide_mrt(CT* f, CT rho, CT ux, CT uy, CT uz, CT nu)
-{
-    CT Pxx, Pyy, Pzz, Pxy, Pxz, Pyz, tr;
-    mrt_moments<CT>(f, rho, ux, uy, uz, nu, Pxx, Pyy, Pzz, Pxy, Pxz, Pyz, tr);
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int cx = cxq(q), cy = cyq(q), cz = czq(q);
-        const int c2 = cx * cx + cy * cy + cz * cz;
-        const CT cu = CT(cx) * ux + CT(cy) * uy + CT(cz) * uz;
-        const CT pp = CT(cx * cx) * Pxx + CT(cy * cy) * Pyy + CT(cz * cz) * Pzz
-                      + CT(2) * (CT(cx * cy) * Pxy + CT(cx * cz) * Pxz + CT(cy * cz) * Pyz);
-        f[q] = weight<CT>(q) * (rho * (CT(2.5) - CT(1.5) * CT(c2) + CT(3) * cu) + CT(4.5) * pp - CT(1.5) * tr);
-    }
-}
-
-// MRT_LES of one cell in single precision, its rebuild with the planes x = -1 and x = 0 as
-// packed f2 pairs (the terms without c_x are shared by the pair; the x = +1 plane runs
-// scalar)
-__device__ __forceinline__ void collide_mrt_packed(float* f, float rho, float ux, float uy, float uz, float nu)
-{
-    float Pxx, Pyy, Pzz, Pxy, Pxz, Pyz, tr;
-    mrt_moments<float>(f, rho, ux, uy, uz, nu, Pxx, Pyy, Pzz, Pxy, Pxz, Pyz, tr);
-    const f2 rho2(rho, rho), ux0(-ux, 0.f), three(3.0), p45(4.5), tr15(1.5f * tr, 1.5f * tr);
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy)
-#pragma unroll
-        for (int iz = 0; iz < 3; ++iz) {
-            const int cy = iy - 1, cz = iz - 1, j = 3 * iy + iz;
-            const float s_cu = (float)cy * uy + (float)cz * uz;
-            const float s_pp = (float)(cy * cy) * Pyy + (float)(cz * cz) * Pzz + 2.f * (float)(cy * cz) * Pyz;
-            const float x_pp = 2.f * ((float)cy * Pxy + (float)cz * Pxz);
-            const int s_c2 = cy * cy + cz * cz;
-            // x = -1 (c_x^2 = 1) and x = 0
-            const f2 cu = ux0 + f2(s_cu, s_cu);
-            const f2 pp = f2(Pxx - x_pp, 0.f) + f2(s_pp, s_pp);
-            const f2 k(2.5f - 1.5f * (float)(1 + s_c2), 2.5f - 1.5f * (float)s_c2);
-            const f2 w(weight<float>(j), weight<float>(9 + j));
-            const f2 v = w * (mad(rho2, mad(three, cu, k), p45 * pp) - tr15);
-            f[j] = v.v.x;
-            f[9 + j] = v.v.y;
-            // x = +1
-            const float cu1 = ux + s_cu, pp1 = Pxx + x_pp + s_pp;
-            f[18 + j] = weight<float>(18 + j) * (rho * (2.5f - 1.5f * (float)(1 + s_c2) + 3.f * cu1) + 4.5f * pp1 - 1.5f * tr);
-        }
-}
-
-// ---------------------------------------------------------------------------------------
-// KBC (Karlin, Boesch, Chikatamarla 2015), lbm_col_kbc_n.h / lbm_col_kbc_c.h: shear part
-// s = D [+T] [+Q] of raw (N) or central (C) moments, entropic stabiliser gamma,
-// f -= beta (2 ds + gamma dh) - (1-beta) S feq.  Two passes over q keep the per-direction
-// temporaries out of registers.
-// ---------------------------------------------------------------------------------------
-template <class CT>
-struct KbcMom { CT T, Nxz, Nyz, Pxy, Pxz, Pyz, Qxxy, Qxxz, Qxyy, Qyyz, Qxzz, Qyzz, Qxyz; };
-
-template <class CT, bool USE_T, bool USE_Q>
-__device__ __forceinline__ CT kbc_shear(int q, const KbcMom<CT>& m)
-{
-    const int cx = cxq(q), cy = cyq(q), cz = czq(q), nz0 = nnzq(q);
-    CT D = CT(0), T = CT(0), Qv = CT(0);
-    if (nz0 == 1) {
-        if (cx) D = (CT(2) * m.Nxz - m.Nyz) * CT(1.0 / 6.0);
-        if (cy) D = (-m.Nxz + CT(2) * m.Nyz) * CT(1.0 / 6.0);
-        if (cz) D = (-m.Nxz - m.Nyz) * CT(1.0 / 6.0);
-        T = m.T * CT(1.0 / 6.0);
-        if (cx) Qv = CT(-cx) * (m.Qxyy + m.Qxzz) * CT(0.5);
-        if (cy) Qv = CT(-cy) * (m.Qxxy + m.Qyzz) * CT(0.5);
-        if (cz) Qv = CT(-cz) * (m.Qxxz + m.Qyyz) * CT(0.5);
-    } else if (nz0 == 2) {
-        if (!cz) { D = CT(cx * cy) * m.Pxy * CT(0.25); Qv = (CT(cx) * m.Qxyy + CT(cy) * m.Qxxy) * CT(0.25); }
-        if (!cy) { D = CT(cx * cz) * m.Pxz * CT(0.25); Qv = (CT(cx) * m.Qxzz + CT(cz) * m.Qxxz) * CT(0.25); }
-        if (!cx) { D = CT(cy * cz) * m.Pyz * CT(0.25); Qv = (CT(cy) * m.Qyzz + CT(cz) * m.Qyyz) * CT(0.25); }
-    } else if (nz0 == 3) {
-        Qv = CT(cx * cy * cz) * m.Qxyz * CT(0.125);
-    } else {
-        T = -m.T;
-    }
-    return D + (USE_T ? T : CT(0)) + (USE_Q ? Qv : CT(0));
-}
-
-// the entropic stabiliser gamma = 1/beta - (2 - 1/beta) num/den; the reference divides 0/0
-// when dh vanishes identically, where gamma*dh is zero for any finite gamma and the
-// regularised limit 1/beta is taken
-template <class CT>
-__device__ __forceinline__ CT kbc_gamma(CT num, CT den, CT beta)
-{
-    return den != CT(0) ? CT(1) / beta - (CT(2) - CT(1) / beta) * num / den : CT(1) / beta;
-}
-__device__ __forceinline__ f2 kbc_gamma(f2 num, f2 den, f2 beta)
-{
-    return f2(kbc_gamma<float>(num.v.x, den.v.x, beta.v.x), kbc_gamma<float>(num.v.y, den.v.y, beta.v.y));
-}
-
-template <class CT, bool CENTRAL, bool USE_T, bool USE_Q>
-__device__ __forceinline__ void collide_kbc(CT* f, CT rho, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz, CT nu)
-{
-    CT M200 = CT(0), M020 = CT(0), M002 = CT(0), M110 = CT(0), M101 = CT(0), M011 = CT(0), M111 = CT(0);
-    CT M201 = CT(0), M102 = CT(0), M210 = CT(0), M120 = CT(0), M021 = CT(0), M012 = CT(0);
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int cx = cxq(q), cy = cyq(q), cz = czq(q);
-        const CT v = f[q];
-        if (cx) { M200 += v; if (cz) M201 += CT(cz) * v; if (cy) M210 += CT(cy) * v; }
-        if (cy) { M020 += v; if (cz) M021 += CT(cz) * v; if (cx) M120 += CT(cx) * v; }
-        if (cz) { M002 += v; if (cx) M102 += CT(cx) * v; if (cy) M012 += CT(cy) * v; }
-        if (cx && cy) M110 += CT(cx * cy) * v;
-        if (cx && cz) M101 += CT(cx * cz) * v;
-        if (cy && cz) M011 += CT(cy * cz) * v;
-        if (cx && cy && cz) M111 += CT(cx * cy * cz) * v;
-    }
-    const CT cs2 = CT(1.0 / 3.0);
-    KbcMom<CT> m, e;
-    const CT rT = M200 + M020 + M002, rNxz = M200 - M002, rNyz = M020 - M002;
-    if (!CENTRAL) {
-        m = {rT, rNxz, rNyz, M110, M101, M011, M210, M201, M120, M021, M102, M012, M111};
-        e.T = rho * (CT(3) * cs2 + ux * ux + uy * uy + uz * uz);
-        e.Nxz = rho * (ux * ux - uz * uz); e.Nyz = rho * (uy * uy - uz * uz);
-        e.Pxy = rho * ux * uy; e.Pxz = rho * ux * uz; e.Pyz = rho * uy * uz;
-        e.Qxxy = rho * uy * (cs2 + ux * ux); e.Qxxz = rho * uz * (cs2 + ux * ux);
-        e.Qxyy = rho * ux * (cs2 + uy * uy); e.Qyyz = rho * uz * (cs2 + uy * uy);
-        e.Qxzz = rho * ux * (cs2 + uz * uz); e.Qyzz = rho * uy * (cs2 + uz * uz);
-        e.Qxyz = rho * ux * uy * uz;
-    } else {
-        const CT cT = rT - rho * (ux * ux + uy * uy + uz * uz);
-        const CT cNxz = rNxz + rho * (uz * uz - ux * ux), cNyz = rNyz + rho * (uz * uz - uy * uy);
-        const CT cPxy = M110 - rho * ux * uy, cPxz = M101 - rho * ux * uz, cPyz = M011 - rho * uy * uz;
-        m.T = cT; m.Nxz = cNxz; m.Nyz = cNyz; m.Pxy = cPxy; m.Pxz = cPxz; m.Pyz = cPyz;
-        m.Qxxy = M210 - CT(1.0 / 3.0) * (CT(6) * ux * cPxy + uy * (CT(3) * ux * ux + CT(2) * cNxz - cNyz + cT));
-        m.Qxxz = M201 - CT(1.0 / 3.0) * (CT(6) * ux * cPxz + uz * (CT(3) * ux * ux + CT(2) * cNxz - cNyz + cT));
-        m.Qxyy = M120 - CT(1.0 / 3.0) * (CT(6) * uy * cPxy + ux * (CT(3) * uy * uy + CT(2) * cNyz - cNxz + cT));
-        m.Qyyz = M021 - CT(1.0 / 3.0) * (CT(6) * uy * cPyz + uz * (CT(3) * uy * uy + CT(2) * cNyz - cNxz + cT));
-        m.Qxzz = M102 - CT(1.0 / 3.0) * (CT(6) * uz * cPxz + ux * (CT(3) * uz * uz - cNyz - cNxz + cT));
-        m.Qyzz = M012 - CT(1.0 / 3.0) * (CT(6) * uz * cPyz + uy * (CT(3) * uz * uz - cNyz - cNxz + cT));
-        m.Qxyz = M111 - ux * cPyz - uy * cPxz - uz * cPxy - ux * uy * uz;
-        const CT z = CT(0);
-        e = {rho * CT(3) * cs2, z, z, z, z, z, z, z, z, z, z, z, z};
-    }
-    const FactEq<CT> E(ux, uy, uz);
-    const CT beta = CT(1) / (CT(2) * nu / cs2 + CT(1));
-    // the shear part is linear in the moments: Delta s_q = s_q(m) - s_q(m_eq) = s_q(m - m_eq)
-    const KbcMom<CT> dm = {m.T - e.T, m.Nxz - e.Nxz, m.Nyz - e.Nyz, m.Pxy - e.Pxy, m.Pxz - e.Pxz, m.Pyz - e.Pyz,
-                           m.Qxxy - e.Qxxy, m.Qxxz - e.Qxxz, m.Qxyy - e.Qxyy, m.Qyyz - e.Qyyz, m.Qxzz - e.Qxzz,
-                           m.Qyzz - e.Qyzz, m.Qxyz - e.Qxyz};
-    CT num = CT(0), den = CT(0);
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const CT feq = E(q, rho);
-        const CT ds = kbc_shear<CT, USE_T, USE_Q>(q, dm);
-        const CT dh = f[q] - feq - ds;
-        const CT ifeq = CT(1) / feq;
-        num += ds * dh * ifeq;
-        den += dh * dh * ifeq;
-    }
-    const CT gamma = kbc_gamma(num, den, beta);
-    const CT ir = CT(1) / rho;
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const CT feq = E(q, rho);
-        const CT ds = kbc_shear<CT, USE_T, USE_Q>(q, dm);
-        const CT dh = f[q] - feq - ds;
-        f[q] -= beta * (CT(2) * ds + gamma * dh) - (CT(1) - beta) * force_src<CT>(q, ir, ux, uy, uz, fx, fy, fz) * feq;
-    }
-}
-
-template <class CT, class PT>
-__device__ __forceinline__ CT local_nu(const CT* f, CT rho, CT ux, CT uy, CT uz, const CYParams<PT>& p, CT* S);
-
-// one collision; with `cy` the shear viscosity is the local Carreau-Yasuda one.  CT is
-// the arithmetic type (f2: two cells at once), PT that of the viscosity-law parameters
-template <class CT, int COL, class PT = CT>
-__device__ __forceinline__ void collide(CT* f, CT rho, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz, CT nu,
-                                        const CYParams<PT>* cy = nullptr, CT* S = nullptr)
-{
-    if constexpr (COL != COL_CUM) {
-        if (cy) nu = local_nu<CT, PT>(f, rho, ux, uy, uz, *cy, S);
-    }
-    if constexpr (COL == COL_CUM) collide_cum<CT, PT>(f, rho, ux, uy, uz, nu, cy, S);
-    else if constexpr (COL == COL_MRT) collide_mrt<CT>(f, rho, ux, uy, uz, nu);
-    else if constexpr (COL == COL_BGK) collide_bgk<CT>(f, rho, ux, uy, uz, fx, fy, fz, nu);
-    else {
-        constexpr bool central = COL >= COL_KBC_C1;
-        constexpr int v = central ? COL - COL_KBC_C1 + 1 : COL - COL_KBC_N1 + 1;
-        collide_kbc<CT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(f, rho, ux, uy, uz, fx, fy, fz, nu);
-    }
-}
-
-// density, velocity (u = (j + F/2) / rho) and the collision of one cell's populations.  For
-// the cumulant the first half of the forward transform's z pass sums the populations by
-// column, and the density and momentum come from those sums instead of separate sums over
-// all 27
-// PACK_DT: the storage type of a one-cell step in single precision (0: none), which picks the
-// forms with the planes x = -1, 0 as packed pairs: the cumulant and BGK with every
-// single-precision storage, MRT_LES with 16-bit storage (with FP32 storage, bound by HBM,
-// the packed rebuild measured 1 % slower).  KBC keeps the scalar sums: at its 128 registers
-// the packed ones spill and measured 5 % slower
-template <class CT, int COL, class PT = CT, int PACK_DT = 0>
-__device__ __forceinline__ void step_cell(CT* f, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, CT* S, CT& rho, CT& ux,
-                                          CT& uy, CT& uz)
-{
-    constexpr bool PACK = PACK_DT != 0 && std::is_same<CT, float>::value;
-    if constexpr (COL == COL_CUM && PACK && NNLBM_CUM_PACKED) {
-        step_cell_cum_packed(f, fx, fy, fz, nu, cy, S, rho, ux, uy, uz);
-    } else if constexpr (COL == COL_MRT && PACK && PACK_DT >= 2) {
-        packed_density_velocity(f, fx, fy, fz, rho, ux, uy, uz);
-        if (cy) nu = local_nu<CT, PT>(f, rho, ux, uy, uz, *cy, S);
-        collide_mrt_packed(f, rho, ux, uy, uz, nu);
-    } else if constexpr (COL == COL_BGK && PACK) {
-        packed_density_velocity(f, fx, fy, fz, rho, ux, uy, uz);
-        if (cy) nu = local_nu<CT, PT>(f, rho, ux, uy, uz, *cy, S);
-        collide_bgk_packed(f, rho, ux, uy, uz, fx, fy, fz, nu);
-    } else if constexpr (COL == COL_CUM) {
-        cum_columns<CT>(f);
-        cum_density_velocity<CT>(f, fx, fy, fz, rho, ux, uy, uz);
-        collide_cum_columns<CT, PT>(f, rho, ux, uy, uz, nu, cy, S);
-    } else {
-        density_velocity<CT>(f, fx, fy, fz, rho, ux, uy, uz);
-        collide<CT, COL, PT>(f, rho, ux, uy, uz, fx, fy, fz, nu, cy, S);
-    }
-}
-
-// ---------------------------------------------------------------------------------------
 // Carreau-Yasuda local viscosity from the non-equilibrium second moments:
 // Pi = sum f (c-u)(c-u) - rho/3 I, S = -3/(2 rho tau) Pi, gamma_dot = sqrt(2 S:S),
 // nu = nu_inf + (nu0-nu_inf)(1 + (lambda gamma_dot)^a)^((n-1)/a), tau = 3 nu + 1/2, solved by
@@ -806,12 +161,11 @@ __device__ __forceinline__ void step_cell(CT* f, CT fx, CT fy, CT fz, CT nu, con
 template <class CT>
 struct CYParams { CT nu_inf, nu0, lam, a, n; };
 
-// from the central second moments Cxx.. (not yet reduced by rho/3 on the diagonal)
+// from the central second moments, those on the diagonal reduced by rho/3 (Pxx ..)
 template <class CT>
-__device__ __forceinline__ CT cy_nu_from_central(CT Cxx, CT Cyy, CT Czz, CT Cxy, CT Cxz, CT Cyz, CT rho, const CYParams<CT>& p,
+__device__ __forceinline__ CT cy_nu_from_central(CT Pxx, CT Pyy, CT Pzz, CT Cxy, CT Cxz, CT Cyz, CT rho, const CYParams<CT>& p,
                                                  CT* S)
 {
-    const CT Pxx = Cxx - rho * CT(1.0 / 3.0), Pyy = Cyy - rho * CT(1.0 / 3.0), Pzz = Czz - rho * CT(1.0 / 3.0);
     const CT pn = dsqrt<CT>(Pxx * Pxx + Pyy * Pyy + Pzz * Pzz + CT(2) * (Cxy * Cxy + Cxz * Cxz + Cyz * Cyz));
     const CT K = CT(3) * CT(1.4142135623730951) * pn / (CT(2) * rho);
     CT tau = CT(3) * p.nu0 + CT(0.5);
@@ -839,11 +193,10 @@ __device__ __forceinline__ CT cy_nu_from_central(CT Cxx, CT Cyy, CT Czz, CT Cxy,
 
 // two cells at once: the same Newton solve in packed arithmetic; the powers, square roots
 // and divisions run per half, and a half whose strain is zero keeps tau = 3 nu0 + 1/2
-__device__ __forceinline__ f2 cy_nu_from_central(f2 Cxx, f2 Cyy, f2 Czz, f2 Cxy, f2 Cxz, f2 Cyz, f2 rho,
+__device__ __forceinline__ f2 cy_nu_from_central(f2 Pxx, f2 Pyy, f2 Pzz, f2 Cxy, f2 Cxz, f2 Cyz, f2 rho,
                                                  const CYParams<float>& p, f2* S)
 {
     const f2 third(1.0 / 3.0), half(0.5), three(3.0), one(1.0);
-    const f2 Pxx = Cxx - rho * third, Pyy = Cyy - rho * third, Pzz = Czz - rho * third;
     const f2 pn = dsqrt<f2>(Pxx * Pxx + Pyy * Pyy + Pzz * Pzz + f2(2.0) * (Cxy * Cxy + Cxz * Cxz + Cyz * Cyz));
     const f2 K = three * f2(1.4142135623730951) * pn / (f2(2.0) * rho);
     const f2 tau0 = three * f2(p.nu0) + half;
@@ -873,30 +226,652 @@ __device__ __forceinline__ f2 cy_nu_from_central(f2 Cxx, f2 Cyy, f2 Czz, f2 Cxy,
     return (tau - half) * third;
 }
 
-// the same from the populations: raw second moments by additions only (c in {-1,0,1}),
-// shifted to central ones with the raw momentum j: C_ab = M_ab - u_a j_b - u_b j_a + rho u_a u_b
-template <class CT, class PT>
-__device__ __forceinline__ CT local_nu(const CT* f, CT rho, CT ux, CT uy, CT uz, const CYParams<PT>& p, CT* S)
+// ---------------------------------------------------------------------------------------
+// The collisions work on the stored values themselves: g_q = (f_q - w_q) sc for F32 (sc = 1),
+// FP16 and BF16 storage, f_q for FP64 (DT = 0).  Every moment is linear in them, so the
+// weights and the storage scale meet a handful of moments (or the factors of the equilibrium)
+// instead of each of the 27 populations on the way in and out, and a moment of g carries no
+// rounding of the rest state.  Against populations shifted and scaled one by one, with the
+// moments summed per use, this halves the instructions of a step.
+//
+// PLANES (one cell in single precision): the planes x = -1 and x = 0 run as f2 pairs on the
+// packed FP32 pipe, the plane x = +1 scalar.
+// ---------------------------------------------------------------------------------------
+// the moments of order <= 2 in (y, z), and 21, 12, of the 9 populations 3 iy + iz of one x
+// plane: 17 additions (19 with the third order)
+template <class V>
+struct PlaneMom { V a00, a10, a01, a20, a02, a11, a21, a12; };
+template <class V>
+__device__ __forceinline__ PlaneMom<V> plane_moments(const V* g)
 {
-    CT Mxx = CT(0), Myy = CT(0), Mzz = CT(0), Mxy = CT(0), Mxz = CT(0), Myz = CT(0), jx = CT(0), jy = CT(0), jz = CT(0);
+    V s[3], d[3], c[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        s[i] = g[3 * i + 2] + g[3 * i];
+        d[i] = g[3 * i + 2] - g[3 * i];
+        c[i] = s[i] + g[3 * i + 1];
+    }
+    PlaneMom<V> p;
+    p.a20 = c[2] + c[0];
+    p.a00 = p.a20 + c[1];
+    p.a10 = c[2] - c[0];
+    p.a21 = d[2] + d[0];
+    p.a01 = p.a21 + d[1];
+    p.a11 = d[2] - d[0];
+    p.a02 = (s[2] + s[0]) + s[1];
+    p.a12 = s[2] - s[0];
+    return p;
+}
+__device__ __forceinline__ PlaneMom<float> plane_half(const PlaneMom<f2>& p, int h)
+{
+    auto v = [h](f2 a) { return h ? a.v.y : a.v.x; };
+    return {v(p.a00), v(p.a10), v(p.a01), v(p.a20), v(p.a02), v(p.a11), v(p.a21), v(p.a12)};
+}
+
+// raw moments of the stored values: r = sum g, j = sum c g, second order, and the third order
+// that KBC reads
+template <class CT>
+struct Moments {
+    CT r, jx, jy, jz, xx, yy, zz, xy, xz, yz, xxy, xxz, xyy, yyz, xzz, yzz, xyz;
+};
+template <class CT>
+__device__ __forceinline__ Moments<CT> moments_of_planes(const PlaneMom<CT>& m, const PlaneMom<CT>& z, const PlaneMom<CT>& p)
+{
+    Moments<CT> M;
+    M.xx = p.a00 + m.a00;
+    M.r = M.xx + z.a00;
+    M.jx = p.a00 - m.a00;
+    M.xxy = p.a10 + m.a10;
+    M.jy = M.xxy + z.a10;
+    M.xy = p.a10 - m.a10;
+    M.xxz = p.a01 + m.a01;
+    M.jz = M.xxz + z.a01;
+    M.xz = p.a01 - m.a01;
+    M.yy = (p.a20 + m.a20) + z.a20;
+    M.xyy = p.a20 - m.a20;
+    M.zz = (p.a02 + m.a02) + z.a02;
+    M.xzz = p.a02 - m.a02;
+    M.yz = (p.a11 + m.a11) + z.a11;
+    M.xyz = p.a11 - m.a11;
+    M.yyz = (p.a21 + m.a21) + z.a21;
+    M.yzz = (p.a12 + m.a12) + z.a12;
+    return M;
+}
+template <class CT, bool PLANES>
+__device__ __forceinline__ Moments<CT> raw_moments(const CT* g)
+{
+    if constexpr (PLANES) {
+        f2 pair[9];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) pair[j] = f2(g[j], g[9 + j]);
+        const PlaneMom<f2> p01 = plane_moments<f2>(pair);
+        return moments_of_planes<float>(plane_half(p01, 0), plane_half(p01, 1), plane_moments<float>(g + 18));
+    } else {
+        return moments_of_planes<CT>(plane_moments<CT>(g), plane_moments<CT>(g + 9), plane_moments<CT>(g + 18));
+    }
+}
+
+// what a collision starts from: density (dr = rho - 1 with shifted storage, rho itself with
+// FP64), u = (j + F/2) / rho, its momentum m = j + F/2, the raw moments (in units of f; the
+// second moments on the diagonal less their rest value 1/3 with shifted storage)
+template <class CT>
+struct CellState {
+    Moments<CT> M;
+    CT dr, rho, ir, mx, my, mz, ux, uy, uz;
+};
+template <class CT, int DT, bool PLANES, bool THIRD>
+__device__ __forceinline__ CellState<CT> cell_state(const CT* g, CT fx, CT fy, CT fz, CT isc)
+{
+    CellState<CT> c;
+    c.M = raw_moments<CT, PLANES>(g);
+    if constexpr (DT >= 2) {
+        Moments<CT>& M = c.M;
+        M.r = M.r * isc; M.jx = M.jx * isc; M.jy = M.jy * isc; M.jz = M.jz * isc;
+        M.xx = M.xx * isc; M.yy = M.yy * isc; M.zz = M.zz * isc;
+        M.xy = M.xy * isc; M.xz = M.xz * isc; M.yz = M.yz * isc;
+        if constexpr (THIRD) {
+            M.xxy = M.xxy * isc; M.xxz = M.xxz * isc; M.xyy = M.xyy * isc; M.yyz = M.yyz * isc;
+            M.xzz = M.xzz * isc; M.yzz = M.yzz * isc; M.xyz = M.xyz * isc;
+        }
+    }
+    c.dr = c.M.r;
+    c.rho = DT == 0 ? c.dr : c.dr + CT(1);
+    c.ir = CT(1) / c.rho;
+    c.mx = mad(CT(0.5), fx, c.M.jx);
+    c.my = mad(CT(0.5), fy, c.M.jy);
+    c.mz = mad(CT(0.5), fz, c.M.jz);
+    c.ux = c.mx * c.ir;
+    c.uy = c.my * c.ir;
+    c.uz = c.mz * c.ir;
+    return c;
+}
+
+// central second moments (about u) with rho/3 taken off the diagonal:
+// C_ab = M_ab - u_a j_b - u_b j_a + rho u_a u_b with j = rho u - F/2
+template <class CT>
+struct Central { CT xx, yy, zz, xy, xz, yz; };
+template <class CT>
+__device__ __forceinline__ Central<CT> central_moments(const CellState<CT>& c, CT fx, CT fy, CT fz)
+{
+    const CT third = c.dr * CT(1.0 / 3.0);
+    Central<CT> C;
+    C.xx = mad(-c.ux, c.M.jx - CT(0.5) * fx, c.M.xx - third);
+    C.yy = mad(-c.uy, c.M.jy - CT(0.5) * fy, c.M.yy - third);
+    C.zz = mad(-c.uz, c.M.jz - CT(0.5) * fz, c.M.zz - third);
+    C.xy = mad(-c.uy, c.M.jx, mad(c.ux, CT(0.5) * fy, c.M.xy));
+    C.xz = mad(-c.uz, c.M.jx, mad(c.ux, CT(0.5) * fz, c.M.xz));
+    C.yz = mad(-c.uz, c.M.jy, mad(c.uy, CT(0.5) * fz, c.M.yz));
+    return C;
+}
+
+// ---------------------------------------------------------------------------------------
+// cumulant collision (Geier et al. 2015) with the reference configuration of
+// solver/lbm3d/lbm_col_cum.h:166-282: shear rate omega1 = 1/(3 nu + 1/2), every other rate
+// 1, A = B = 0, no limiter.  With those rates all cumulants of order >= 3 are reset to
+// zero: the collision reads the moments up to second order only, and the post-collision
+// central moments of order 4 and 6 are those of a Gaussian (G2015 Eq 81-84 with the odd
+// orders zero; the sixth, collected, is
+// s222 = (s200 s020 s002 + 2 (s200 s011^2 + s020 s101^2 + s002 s110^2) + 8 s110 s101 s011) / rho^2).
+// The first-order ones are F/2.
+//
+// The populations are rebuilt axis by axis: central -> raw moments (r1 = k1 + u k0,
+// r2 = k2 + u (k1 + r1)), the rest state's raw moments taken off, raw moments -> populations
+// (p = (r2 + r1)/2, m = (r2 - r1)/2, z = r0 - r2).  Each moment carries a factor 1/2 per axis
+// of non-zero order from the start, so that no halving is left: 3 operations a triple
+// and direction.
+// ---------------------------------------------------------------------------------------
+template <class V>
+__device__ __forceinline__ void to_raw(V u, V uh, V k0, V& k1, V& k2)
+{
+    const V r1 = mad(uh, k0, k1);
+    k2 = mad(u, k1 + r1, k2);
+    k1 = r1;
+}
+template <class V>
+__device__ __forceinline__ void to_pops(V& a, V& b, V& c)
+{
+    const V p = c + b, m = c - b;
+    b = mad(V(-2.0), c, a);
+    a = m;
+    c = p;
+}
+
+// scaled central moments of a cell after the collision, times the storage scale: the halves
+// and quarters of the second order (x = s200/2, a = s110/4, ...) and the density
+template <class CT>
+struct CumPost { CT r, x, y, z, a, b, c; };  // a: 110, b: 101, c: 011
+
+// the raw moments k[i][j][l] of the post-collision state (x pass; the orders that vanish are
+// left out of the arithmetic)
+template <class CT>
+__device__ __forceinline__ void cum_x_raw(const CumPost<CT>& s, CT irs, CT ux, CT fx, CT fy, CT fz, CT (&k)[3][3][3])
+{
+    const CT uh = CT(0.5) * ux;
+    const CT four = CT(4), eight = CT(8);
+    // fourth and sixth order from products
+    const CT s211 = mad(s.x, s.c, four * (s.a * s.b)) * irs;
+    const CT s121 = mad(s.y, s.b, four * (s.a * s.c)) * irs;
+    const CT s112 = mad(s.z, s.a, four * (s.b * s.c)) * irs;
+    const CT s220 = mad(s.x, s.y, eight * (s.a * s.a)) * irs;
+    const CT s202 = mad(s.x, s.z, eight * (s.b * s.b)) * irs;
+    const CT s022 = mad(s.y, s.z, eight * (s.c * s.c)) * irs;
+    const CT s222 = mad(s.x, s022, eight * mad(s.b, s121, s.a * s112)) * irs;
+    // first order F/2 (times 1/2)
+    k[0][0][0] = s.r; k[1][0][0] = CT(0.25) * fx; k[2][0][0] = s.x;
+    to_raw<CT>(ux, uh, k[0][0][0], k[1][0][0], k[2][0][0]);
+    // orders (., 1, 0) and (., 0, 1): no k2
+    k[0][1][0] = CT(0.25) * fy;
+    k[1][1][0] = mad(uh, k[0][1][0], s.a);
+    k[2][1][0] = ux * (s.a + k[1][1][0]);
+    k[0][0][1] = CT(0.25) * fz;
+    k[1][0][1] = mad(uh, k[0][0][1], s.b);
+    k[2][0][1] = ux * (s.b + k[1][0][1]);
+    // orders (., 2, 0), (., 0, 2), (., 1, 1), (., 2, 2): no k1
+    auto even = [&](int j, int l, CT k0, CT k2) {
+        k[0][j][l] = k0;
+        k[1][j][l] = uh * k0;
+        k[2][j][l] = mad(ux, k[1][j][l], k2);
+    };
+    even(2, 0, s.y, s220);
+    even(0, 2, s.z, s202);
+    even(1, 1, s.c, s211);
+    even(2, 2, s022, s222);
+    // orders (., 2, 1) and (., 1, 2): k1 only
+    k[0][2][1] = CT(0); k[1][2][1] = s121; k[2][2][1] = ux * (s121 + s121);
+    k[0][1][2] = CT(0); k[1][1][2] = s112; k[2][1][2] = ux * (s112 + s112);
+}
+
+template <class CT, int DT, bool PLANES, class PT>
+__device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy,
+                                            CT* S, CT sc, CT isc)
+{
+    const Central<CT> C = central_moments<CT>(c, fx, fy, fz);
+    if (cy) nu = cy_nu_from_central(C.xx, C.yy, C.zz, C.xy, C.xz, C.yz, c.rho, *cy, S);
+    const CT om = CT(1) / (CT(3) * nu + CT(0.5));
+    // relaxation (lbm_col_cum.h:205-235 with omega2 = 1): the shear parts by omega1, the trace
+    // to rho; all times the storage scale
+    const CT k = DT >= 2 ? (CT(1) - om) * sc : CT(1) - om;
+    const CT irs = DT >= 2 ? c.ir * isc : c.ir;
+    if constexpr (DT >= 2) { fx = fx * sc; fy = fy * sc; fz = fz * sc; }
+    const CT e1 = k * (C.xx - C.yy), e2 = k * (C.xx - C.zz), kq = CT(0.25) * k;
+    CumPost<CT> s;
+    s.r = DT >= 2 ? c.rho * sc : c.rho;
+    s.x = CT(1.0 / 6.0) * ((e1 + e2) + s.r);
+    s.y = mad(CT(-0.5), e1, s.x);
+    s.z = mad(CT(-0.5), e2, s.x);
+    s.a = kq * C.xy;
+    s.b = kq * C.xz;
+    s.c = kq * C.yz;
+    CT m[3][3][3];
+    cum_x_raw<CT>(s, irs, c.ux, fx, fy, fz, m);
+    const CT w1 = DT >= 2 ? sc * CT(1.0 / 6.0) : CT(1.0 / 6.0);
+    const CT w2 = w1 * CT(1.0 / 6.0), w3 = w2 * CT(1.0 / 6.0);
+    // the rest state's raw moments (times 1/2 per axis of order 2) off plane m[i] (order i in x)
+    const CT r0 = DT >= 2 ? c.dr * sc : c.dr;
+    if constexpr (PLANES) {
+        // orders i = 0, 1 in x as pairs, i = 2 scalar
+        f2 P[3][3];
+        float Q[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) { P[j][l] = f2(m[0][j][l], m[1][j][l]); Q[j][l] = m[2][j][l]; }
+        const f2 uy2(c.uy, c.uy), uyh2(0.5f * c.uy, 0.5f * c.uy), uz2(c.uz, c.uz), uzh2(0.5f * c.uz, 0.5f * c.uz);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            to_raw<f2>(uy2, uyh2, P[0][l], P[1][l], P[2][l]);
+            to_raw<float>(uy2.v.x, uyh2.v.x, Q[0][l], Q[1][l], Q[2][l]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            to_raw<f2>(uz2, uzh2, P[j][0], P[j][1], P[j][2]);
+            to_raw<float>(uz2.v.x, uzh2.v.x, Q[j][0], Q[j][1], Q[j][2]);
+        }
+        P[0][0].v.x = r0;
+        P[2][0].v.x -= w1; P[0][2].v.x -= w1; Q[0][0] -= w1;
+        P[2][2].v.x -= w2; Q[2][0] -= w2; Q[0][2] -= w2;
+        Q[2][2] -= w3;
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            to_pops<f2>(P[0][l], P[1][l], P[2][l]);
+            to_pops<float>(Q[0][l], Q[1][l], Q[2][l]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            to_pops<f2>(P[j][0], P[j][1], P[j][2]);
+            to_pops<float>(Q[j][0], Q[j][1], Q[j][2]);
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                float a = P[j][l].v.x, b = P[j][l].v.y, d = Q[j][l];
+                to_pops<float>(a, b, d);
+                g[3 * j + l] = a; g[9 + 3 * j + l] = b; g[18 + 3 * j + l] = d;
+            }
+        }
+    } else {
+        const CT uyh = CT(0.5) * c.uy, uzh = CT(0.5) * c.uz;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int l = 0; l < 3; ++l) to_raw<CT>(c.uy, uyh, m[i][0][l], m[i][1][l], m[i][2][l]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) to_raw<CT>(c.uz, uzh, m[i][j][0], m[i][j][1], m[i][j][2]);
+        }
+        if constexpr (DT != 0) {
+            m[0][0][0] = r0;
+            m[2][0][0] -= w1; m[0][2][0] -= w1; m[0][0][2] -= w1;
+            m[2][2][0] -= w2; m[2][0][2] -= w2; m[0][2][2] -= w2;
+            m[2][2][2] -= w3;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int l = 0; l < 3; ++l) to_pops<CT>(m[i][0][l], m[i][1][l], m[i][2][l]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) to_pops<CT>(m[i][j][0], m[i][j][1], m[i][j][2]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                to_pops<CT>(m[0][j][l], m[1][j][l], m[2][j][l]);
+                g[3 * j + l] = m[0][j][l]; g[9 + 3 * j + l] = m[1][j][l]; g[18 + 3 * j + l] = m[2][j][l];
+            }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// factorised equilibrium of the BGK / KBC schemes (lbm_col_bgk.h:43-53, 85-111):
+// feq_q = -rho X_cx Y_cy Z_cz with Xz = u^2 - 2/3, Xp = -(u^2 + u + 1/3)/2, Xm = Xp + u
+// ---------------------------------------------------------------------------------------
+template <class CT>
+struct FactEq {
+    CT X[3], Y[3], Z[3];
+    __device__ __forceinline__ FactEq(CT ux, CT uy, CT uz)
+    {
+        X[1] = mad(ux, ux, CT(1.0 / 3.0) - CT(1)); X[2] = CT(-0.5) * (X[1] + CT(1) + ux); X[0] = X[2] + ux;
+        Y[1] = mad(uy, uy, CT(1.0 / 3.0) - CT(1)); Y[2] = CT(-0.5) * (Y[1] + CT(1) + uy); Y[0] = Y[2] + uy;
+        Z[1] = mad(uz, uz, CT(1.0 / 3.0) - CT(1)); Z[2] = CT(-0.5) * (Z[1] + CT(1) + uz); Z[0] = Z[2] + uz;
+    }
+};
+
+// forcing source S_q of lbm_col_bgk.h:57-83
+template <class CT>
+__device__ __forceinline__ CT force_src(int q, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
+{
+    return (CT(3) * ((CT(cxq(q)) - ux) * fx + (CT(cyq(q)) - uy) * fy + (CT(czq(q)) - uz) * fz)) * ir;
+}
+// whether a cell carries a body force (the source terms of BGK and KBC vanish without one)
+__device__ __forceinline__ bool any_force(float fx, float fy, float fz) { return fx != 0.f || fy != 0.f || fz != 0.f; }
+__device__ __forceinline__ bool any_force(double fx, double fy, double fz) { return fx != 0.0 || fy != 0.0 || fz != 0.0; }
+__device__ __forceinline__ bool any_force(f2 fx, f2 fy, f2 fz)
+{
+    return any_force(fx.v.x, fy.v.x, fz.v.x) || any_force(fx.v.y, fy.v.y, fz.v.y);
+}
+// g_q += k S_q feq_q sc for every direction (rs = rho sc), out of line on a copy, so that the
+// path without a force keeps its populations in registers
+template <class CT>
+__device__ __noinline__ void add_force_all(CT* g, CT k, CT rs, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
+{
+    const FactEq<CT> E(ux, uy, uz);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
-        const int cx = cxq(q), cy = cyq(q), cz = czq(q);
-        const CT v = f[q];
-        if (cx) { Mxx += v; if (cx > 0) jx += v; else jx -= v; }
-        if (cy) { Myy += v; if (cy > 0) jy += v; else jy -= v; }
-        if (cz) { Mzz += v; if (cz > 0) jz += v; else jz -= v; }
-        if (cx * cy > 0) Mxy += v; else if (cx * cy < 0) Mxy -= v;
-        if (cx * cz > 0) Mxz += v; else if (cx * cz < 0) Mxz -= v;
-        if (cy * cz > 0) Myz += v; else if (cy * cz < 0) Myz -= v;
+        const CT feq = -rs * E.X[q / 9] * E.Y[(q / 3) % 3] * E.Z[q % 3];
+        g[q] += k * force_src<CT>(q, ir, ux, uy, uz, fx, fy, fz) * feq;
     }
-    const CT Cxx = Mxx - CT(2) * ux * jx + rho * ux * ux;
-    const CT Cyy = Myy - CT(2) * uy * jy + rho * uy * uy;
-    const CT Czz = Mzz - CT(2) * uz * jz + rho * uz * uz;
-    const CT Cxy = Mxy - ux * jy - uy * jx + rho * ux * uy;
-    const CT Cxz = Mxz - ux * jz - uz * jx + rho * ux * uz;
-    const CT Cyz = Myz - uy * jz - uz * jy + rho * uy * uz;
-    return cy_nu_from_central(Cxx, Cyy, Czz, Cxy, Cxz, Cyz, rho, p, S);
+}
+template <class CT>
+__device__ __forceinline__ void add_force(CT* g, CT k, CT rs, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
+{
+    CT t[27];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) t[q] = g[q];
+    add_force_all<CT>(t, k, rs, ir, ux, uy, uz, fx, fy, fz);
+#pragma unroll
+    for (int q = 0; q < 27; ++q) g[q] = t[q];
+}
+
+// The equilibrium of BGK and KBC in the units of the stored values, geq_q = (feq_q - w_q) s
+// (feq_q s with FP64 storage).  Per axis the factor is its weight W (1/6, 2/3, 1/6) plus a
+// deviation A ((u^2 - u)/2, -u^2, (u^2 + u)/2); the product less w_q is collected as
+//   X_i b_jl + T_i,n,   b_jl = A_j F_l + W_j A_l,  F = W + A,  X_i = s rho F_i,
+//   T_i,n = (s rho A_i + s (rho - 1) W_i) W_j W_l
+// so that nothing of the size of w_q is ever rounded and taken off again (a population's
+// error would then be a bias of the density, the same in every step)
+template <class CT, int DT>
+struct GridEq {
+    CT X[3], T[3][3], b[3][3];
+    __device__ static __forceinline__ void axis(CT u, CT* A, CT* F)
+    {
+        const CT h = CT(0.5) * u, uu = u * u;
+        A[1] = -uu;
+        A[2] = mad(h, u, h);
+        A[0] = mad(h, u, -h);
+        F[1] = CT(2.0 / 3.0) - uu;
+        F[2] = CT(1.0 / 6.0) + A[2];
+        F[0] = CT(1.0 / 6.0) + A[0];
+    }
+    // s rho, s (rho - 1)
+    __device__ __forceinline__ GridEq(CT ux, CT uy, CT uz, CT rs, CT drs, CT* Fx, CT* Fy, CT* Fz)
+    {
+        CT Ax[3], Ay[3], Az[3];
+        axis(ux, Ax, Fx);
+        axis(uy, Ay, Fy);
+        axis(uz, Az, Fz);
+        const CT W[3] = {CT(1.0 / 6.0), CT(2.0 / 3.0), CT(1.0 / 6.0)};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            X[i] = rs * Fx[i];
+            if constexpr (DT != 0) {
+                const CT t = mad(rs, Ax[i], drs * W[i]);
+                T[i][0] = t * CT(4.0 / 9.0);
+                T[i][1] = t * CT(1.0 / 9.0);
+                T[i][2] = t * CT(1.0 / 36.0);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) b[j][l] = DT == 0 ? Fy[j] * Fz[l] : mad(Ay[j], Fz[l], W[j] * Az[l]);
+    }
+    __device__ __forceinline__ CT operator()(int i, int j, int l) const
+    {
+        return DT == 0 ? X[i] * b[j][l] : mad(X[i], b[j][l], T[i][(j != 1) + (l != 1)]);
+    }
+    // the planes i = 0, 1 as a pair
+    __device__ __forceinline__ f2 pair(int j, int l) const
+    {
+        const int n = (j != 1) + (l != 1);
+        return mad(f2(X[0], X[1]), f2(b[j][l], b[j][l]), f2(T[0][n], T[1][n]));
+    }
+};
+
+// BGK, solver/lbm3d/lbm_col_bgk.h:14-140: g' = (1 - om) g + om geq, the factor om inside geq:
+// two operations a direction
+template <class CT, int DT, bool PLANES>
+__device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, CT sc)
+{
+    const CT om = CT(1) / (CT(3) * nu + CT(0.5));
+    const CT rs = DT >= 2 ? c.rho * sc : c.rho, drs = DT >= 2 ? c.dr * sc : c.dr;
+    CT Fx[3], Fy[3], Fz[3];
+    const GridEq<CT, DT> E(c.ux, c.uy, c.uz, om * rs, om * drs, Fx, Fy, Fz);
+    const CT k = CT(1) - om;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            const int q = 3 * j + l;
+            if constexpr (PLANES) {
+                const f2 v = mad(f2(k, k), f2(g[q], g[9 + q]), E.pair(j, l));
+                g[q] = v.v.x;
+                g[9 + q] = v.v.y;
+            } else {
+                g[q] = mad(k, g[q], E(0, j, l));
+                g[9 + q] = mad(k, g[9 + q], E(1, j, l));
+            }
+            g[18 + q] = mad(k, g[18 + q], E(2, j, l));
+        }
+    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - CT(0.5) * om, rs, c.ir, c.ux, c.uy, c.uz, fx, fy, fz);
+}
+
+// ---------------------------------------------------------------------------------------
+// MRT_LES, solver/lbm3d/lbm_col_mrt.h:12-78: second moments relaxed with a Smagorinsky rate,
+// everything rebuilt as w_q [rho (1 + 3 c.u) + 9/2 (c c - I/3) : (P - rho I/3)] form.  With P
+// and rho less their rest values the brackets give (f - w) directly; opposite directions
+// share their even part and differ by the sign of the odd one (3 rho c.u).
+// ---------------------------------------------------------------------------------------
+template <class CT, int DT>
+__device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu, CT sc)
+{
+    const Moments<CT>& M = c.M;
+    const CT third = c.dr * CT(1.0 / 3.0);
+    const CT nxx = mad(-c.mx, c.ux, M.xx - third), nyy = mad(-c.my, c.uy, M.yy - third), nzz = mad(-c.mz, c.uz, M.zz - third);
+    const CT nxy = mad(-c.mx, c.uy, M.xy), nxz = mad(-c.mx, c.uz, M.xz), nyz = mad(-c.my, c.uz, M.yz);
+    const CT Qs = CT(2) * (nxx * nxx + nyy * nyy + nzz * nzz + CT(2) * (nxy * nxy + nxz * nxz + nyz * nyz));
+    const CT tau = CT(3) * nu + CT(0.5);
+    const CT om = CT(2) / (dsqrt<CT>(tau * tau + CT(2) * CT(0.0342) * CT(9) * dsqrt<CT>(Qs) * c.ir) + tau);
+    const CT Pxx = mad(-om, nxx, M.xx), Pyy = mad(-om, nyy, M.yy), Pzz = mad(-om, nzz, M.zz);
+    const CT sn = DT >= 2 ? CT(9) * sc : CT(9);
+    const CT xy = sn * mad(-om, nxy, M.xy), xz = sn * mad(-om, nxz, M.xz), yz = sn * mad(-om, nyz, M.yz);
+    const CT s1 = DT >= 2 ? sc : CT(1);
+    // even part: A + B_a per axis with c_a != 0 + 9 c_a c_b P_ab; odd part: 3 rho c.u
+    const CT h = s1 * CT(1.5);
+    const CT A = DT >= 2 ? s1 * mad(CT(-1.5), (Pxx + Pyy) + Pzz, CT(2.5) * c.dr) : mad(CT(-1.5), (Pxx + Pyy) + Pzz, CT(2.5) * c.dr);
+    const CT bx = h * mad(CT(3), Pxx, -c.dr), by = h * mad(CT(3), Pyy, -c.dr), bz = h * mad(CT(3), Pzz, -c.dr);
+    const CT s3 = s1 * CT(3);
+    const CT jx = s3 * c.mx, jy = s3 * c.my, jz = s3 * c.mz;
+    // direction q and its opposite from the even and odd parts
+    auto put = [&](int q, CT e, CT o) {
+        const CT w = CT(weight<double>(q));
+        g[q] = w * (e + o);
+        g[26 - q] = w * (e - o);
+    };
+    g[13] = CT(weight<double>(13)) * A;
+    const CT ax = A + bx, ay = A + by, az = A + bz;
+    put(22, ax, jx); put(16, ay, jy); put(14, az, jz);
+    const CT axy = ax + by, axz = ax + bz, ayz = ay + bz, all = axy + bz;
+    put(25, axy + xy, jx + jy); put(19, axy - xy, jx - jy);
+    put(23, axz + xz, jx + jz); put(21, axz - xz, jx - jz);
+    put(17, ayz + yz, jy + jz); put(15, ayz - yz, jy - jz);
+    put(26, (all + xy) + (xz + yz), (jx + jy) + jz);
+    put(24, (all + xy) - (xz + yz), (jx + jy) - jz);
+    put(20, (all - xy) + (xz - yz), (jx - jy) + jz);
+    put(18, (all - xy) - (xz - yz), (jx - jy) - jz);
+}
+
+// ---------------------------------------------------------------------------------------
+// KBC (Karlin, Boesch, Chikatamarla 2015), lbm_col_kbc_n.h / lbm_col_kbc_c.h: shear part
+// s = D [+T] [+Q] of raw (N) or central (C) moments, entropic stabiliser gamma,
+// f -= beta (2 ds + gamma dh) - (1-beta) S feq.  The shear part is linear in the moments:
+// ds = s(m) - s(m_eq) = s(m - m_eq).  The 27 ds are formed once (opposite directions share
+// their even part) and serve both passes: the products of the stabiliser, whose 1/feq is
+// the product of the inverse factors, and the relaxation
+// g' = g - beta gamma (g - geq) - beta (2 - gamma) ds, geq = (feq - w) sc.
+// ---------------------------------------------------------------------------------------
+// the entropic stabiliser gamma = 1/beta - (2 - 1/beta) num/den; the reference divides 0/0
+// when dh vanishes identically, where gamma*dh is zero for any finite gamma and the
+// regularised limit 1/beta is taken
+template <class CT>
+__device__ __forceinline__ CT kbc_gamma(CT num, CT den, CT beta)
+{
+    return den != CT(0) ? CT(1) / beta - (CT(2) - CT(1) / beta) * num / den : CT(1) / beta;
+}
+
+// ds_q of the moment differences: trace T, normal differences Nxz, Nyz, shears P, third order
+// (its order: xxy xxz xyy yyz xzz yzz xyz), times the storage scale
+template <class CT, bool USE_T, bool USE_Q>
+__device__ __forceinline__ void kbc_shear(CT T, CT Nxz, CT Nyz, CT Pxy, CT Pxz, CT Pyz, const CT* Q, CT* ds)
+{
+    const CT sixth = CT(1.0 / 6.0), q = CT(0.25), h = CT(0.5);
+    CT dx = sixth * (CT(2) * Nxz - Nyz), dy = sixth * (CT(2) * Nyz - Nxz), dz = -(sixth * (Nxz + Nyz));
+    if constexpr (USE_T) {
+        const CT t = sixth * T;
+        dx += t; dy += t; dz += t;
+    }
+    const CT pxy = q * Pxy, pxz = q * Pxz, pyz = q * Pyz;
+    ds[13] = USE_T ? -T : CT(0);
+    if constexpr (USE_Q) {
+        // the odd part of direction q (an opposite one has its negative)
+        auto put = [&](int a, CT e, CT o) { ds[a] = e + o; ds[26 - a] = e - o; };
+        put(22, dx, -(h * (Q[2] + Q[4])));
+        put(16, dy, -(h * (Q[0] + Q[5])));
+        put(14, dz, -(h * (Q[1] + Q[3])));
+        put(25, pxy, q * (Q[2] + Q[0])); put(19, -pxy, q * (Q[2] - Q[0]));
+        put(23, pxz, q * (Q[4] + Q[1])); put(21, -pxz, q * (Q[4] - Q[1]));
+        put(17, pyz, q * (Q[5] + Q[3])); put(15, -pyz, q * (Q[5] - Q[3]));
+        const CT e = CT(0.125) * Q[6];
+        ds[26] = e; ds[24] = -e; ds[20] = -e; ds[18] = e; ds[0] = -e; ds[2] = e; ds[6] = e; ds[8] = -e;
+    } else {
+        ds[22] = dx; ds[4] = dx; ds[16] = dy; ds[10] = dy; ds[14] = dz; ds[12] = dz;
+        ds[25] = pxy; ds[1] = pxy; ds[19] = -pxy; ds[7] = -pxy;
+        ds[23] = pxz; ds[3] = pxz; ds[21] = -pxz; ds[5] = -pxz;
+        ds[17] = pyz; ds[9] = pyz; ds[15] = -pyz; ds[11] = -pyz;
+        ds[0] = ds[2] = ds[6] = ds[8] = ds[18] = ds[20] = ds[24] = ds[26] = CT(0);
+    }
+}
+
+template <class CT, int DT, bool CENTRAL, bool USE_T, bool USE_Q>
+__device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, CT sc)
+{
+    const Moments<CT>& M = c.M;
+    const CT rho = c.rho, ux = c.ux, uy = c.uy, uz = c.uz;
+    const CT xx = ux * ux, yy = uy * uy, zz = uz * uz;
+    const CT cs2 = CT(1.0 / 3.0);
+    CT T, Nxz, Nyz, Pxy, Pxz, Pyz, Q[7];
+    // m - m_eq; the trace of g lacks the rest state's 1, so rho goes in as dr there
+    if constexpr (!CENTRAL) {
+        T = (M.xx + M.yy + M.zz) - c.dr - rho * (xx + yy + zz);
+        Nxz = (M.xx - M.zz) - rho * (xx - zz);
+        Nyz = (M.yy - M.zz) - rho * (yy - zz);
+        Pxy = M.xy - rho * ux * uy; Pxz = M.xz - rho * ux * uz; Pyz = M.yz - rho * uy * uz;
+        Q[0] = M.xxy - rho * uy * (cs2 + xx); Q[1] = M.xxz - rho * uz * (cs2 + xx);
+        Q[2] = M.xyy - rho * ux * (cs2 + yy); Q[3] = M.yyz - rho * uz * (cs2 + yy);
+        Q[4] = M.xzz - rho * ux * (cs2 + zz); Q[5] = M.yzz - rho * uy * (cs2 + zz);
+        Q[6] = M.xyz - rho * ux * uy * uz;
+    } else {
+        T = (M.xx + M.yy + M.zz) - c.dr - rho * (xx + yy + zz);
+        const CT cT = T + rho; // the central trace itself
+        Nxz = (M.xx - M.zz) + rho * (zz - xx);
+        Nyz = (M.yy - M.zz) + rho * (zz - yy);
+        Pxy = M.xy - rho * ux * uy; Pxz = M.xz - rho * ux * uz; Pyz = M.yz - rho * uy * uz;
+        const CT s = CT(6), three = CT(3);
+        Q[0] = M.xxy - cs2 * (s * ux * Pxy + uy * (three * xx + CT(2) * Nxz - Nyz + cT));
+        Q[1] = M.xxz - cs2 * (s * ux * Pxz + uz * (three * xx + CT(2) * Nxz - Nyz + cT));
+        Q[2] = M.xyy - cs2 * (s * uy * Pxy + ux * (three * yy + CT(2) * Nyz - Nxz + cT));
+        Q[3] = M.yyz - cs2 * (s * uy * Pyz + uz * (three * yy + CT(2) * Nyz - Nxz + cT));
+        Q[4] = M.xzz - cs2 * (s * uz * Pxz + ux * (three * zz - Nyz - Nxz + cT));
+        Q[5] = M.yzz - cs2 * (s * uz * Pyz + uy * (three * zz - Nyz - Nxz + cT));
+        Q[6] = M.xyz - ux * Pyz - uy * Pxz - uz * Pxy - ux * uy * uz;
+    }
+    if constexpr (DT >= 2) {
+        T = T * sc; Nxz = Nxz * sc; Nyz = Nyz * sc; Pxy = Pxy * sc; Pxz = Pxz * sc; Pyz = Pyz * sc;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) Q[i] = Q[i] * sc;
+    }
+    CT ds[27];
+    kbc_shear<CT, USE_T, USE_Q>(T, Nxz, Nyz, Pxy, Pxz, Pyz, Q, ds);
+    const CT beta = CT(1) / (CT(6) * nu + CT(1));
+    const CT rs = DT >= 2 ? rho * sc : rho, drs = DT >= 2 ? c.dr * sc : c.dr;
+    CT Fx[3], Fy[3], Fz[3];
+    const GridEq<CT, DT> E(ux, uy, uz, rs, drs, Fx, Fy, Fz);
+    CT num = CT(0), den = CT(0);
+    {
+        const CT iZ[3] = {CT(1) / Fz[0], CT(1) / Fz[1], CT(1) / Fz[2]};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const CT ixy = CT(1) / (E.X[i] * Fy[j]);
+#pragma unroll
+                for (int l = 0; l < 3; ++l) {
+                    const int q = 9 * i + 3 * j + l;
+                    const CT dh = (g[q] - E(i, j, l)) - ds[q];
+                    const CT t = dh * (ixy * iZ[l]);
+                    num = mad(ds[q], t, num);
+                    den = mad(dh, t, den);
+                }
+            }
+    }
+    const CT gamma = kbc_gamma(num, den, beta);
+    const CT bg = beta * gamma, b2 = beta * (CT(2) - gamma);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const int q = 9 * i + 3 * j + l;
+                g[q] = mad(-b2, ds[q], mad(-bg, g[q] - E(i, j, l), g[q]));
+            }
+    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - beta, rs, c.ir, ux, uy, uz, fx, fy, fz);
+}
+
+// density, velocity (u = (j + F/2) / rho) and the collision of one cell's stored values g (or
+// of two cells', CT = f2).  With `cy` the shear viscosity is the local Carreau-Yasuda one and S
+// receives the strain rate.  PT: the type of the viscosity-law parameters
+template <class CT, int COL, int DT, bool PLANES, class PT>
+__device__ __forceinline__ void step_cell(CT* g, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, CT sc, CT isc, CT* S,
+                                          CT& rho, CT& ux, CT& uy, CT& uz)
+{
+    constexpr bool KBC = COL >= COL_KBC_N1 && COL <= COL_KBC_C4;
+    const CellState<CT> c = cell_state<CT, DT, PLANES, KBC>(g, fx, fy, fz, isc);
+    rho = c.rho; ux = c.ux; uy = c.uy; uz = c.uz;
+    if constexpr (COL == COL_CUM) {
+        collide_cum<CT, DT, PLANES, PT>(g, c, fx, fy, fz, nu, cy, S, sc, isc);
+    } else {
+        if (cy) {
+            const Central<CT> C = central_moments<CT>(c, fx, fy, fz);
+            nu = cy_nu_from_central(C.xx, C.yy, C.zz, C.xy, C.xz, C.yz, c.rho, *cy, S);
+        }
+        if constexpr (COL == COL_MRT) {
+            collide_mrt<CT, DT>(g, c, nu, sc);
+        } else if constexpr (COL == COL_BGK) {
+            collide_bgk<CT, DT, PLANES>(g, c, fx, fy, fz, nu, sc);
+        } else {
+            constexpr bool central = COL >= COL_KBC_C1;
+            constexpr int v = central ? COL - COL_KBC_C1 + 1 : COL - COL_KBC_N1 + 1;
+            collide_kbc<CT, DT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(g, c, fx, fy, fz, nu, sc);
+        }
+    }
 }
 
 } // namespace nnlbm
