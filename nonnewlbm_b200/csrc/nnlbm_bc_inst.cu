@@ -53,22 +53,36 @@ __global__ void k_init_macro(const CaseArgs<typename Storage<DT>::CT> a, typenam
     }
 }
 
-void NNLBM_CAT(launch_bc_gather_, NNLBM_DT)(bool odd, dim3 grid, dim3 block, cudaStream_t s, const void* args)
+template <bool ODD, int ARGS>
+static void launch_gather(bool chained, dim3 grid, dim3 block, cudaStream_t s, const GroupArgs<typename Storage<NNLBM_DT>::CT>& g)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, &k_bc_gather<NNLBM_DT, ODD, ARGS>, g);
+}
+void NNLBM_CAT(launch_bc_gather_, NNLBM_DT)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* args)
 {
     using CT = typename Storage<NNLBM_DT>::CT;
     const GroupArgs<CT>& g = *(const GroupArgs<CT>*)args;
     switch (args_mode(g.n_cases)) {
     case ARGS_ONE:
-        if (odd) k_bc_gather<NNLBM_DT, true, ARGS_ONE><<<grid, block, 0, s>>>(g);
-        else k_bc_gather<NNLBM_DT, false, ARGS_ONE><<<grid, block, 0, s>>>(g);
+        if (odd) launch_gather<true, ARGS_ONE>(chained, grid, block, s, g);
+        else launch_gather<false, ARGS_ONE>(chained, grid, block, s, g);
         break;
     case ARGS_PARAM:
-        if (odd) k_bc_gather<NNLBM_DT, true, ARGS_PARAM><<<grid, block, 0, s>>>(g);
-        else k_bc_gather<NNLBM_DT, false, ARGS_PARAM><<<grid, block, 0, s>>>(g);
+        if (odd) launch_gather<true, ARGS_PARAM>(chained, grid, block, s, g);
+        else launch_gather<false, ARGS_PARAM>(chained, grid, block, s, g);
         break;
     default:
-        if (odd) k_bc_gather<NNLBM_DT, true, ARGS_GLOBAL><<<grid, block, 0, s>>>(g);
-        else k_bc_gather<NNLBM_DT, false, ARGS_GLOBAL><<<grid, block, 0, s>>>(g);
+        if (odd) launch_gather<true, ARGS_GLOBAL>(chained, grid, block, s, g);
+        else launch_gather<false, ARGS_GLOBAL>(chained, grid, block, s, g);
     }
 }
 

@@ -28,7 +28,7 @@ namespace nnlbm {
     NNLBM_DECL_STEP(DT, 10)
 NNLBM_DECL_STEP_DT(0) NNLBM_DECL_STEP_DT(1) NNLBM_DECL_STEP_DT(2) NNLBM_DECL_STEP_DT(3)
 #define NNLBM_DECL_AUX(DT)                                                                \
-    void launch_bc_gather_##DT(bool, dim3, dim3, cudaStream_t, const void*);             \
+    void launch_bc_gather_##DT(bool, bool, dim3, dim3, cudaStream_t, const void*);       \
     void launch_refd_velocity_##DT(bool, dim3, dim3, cudaStream_t, const void*);         \
     void launch_refd_stress_##DT(bool, dim3, dim3, cudaStream_t, const void*);           \
     void launch_fill_eq_##DT(const void*, double, double, double, double, cudaStream_t); \
@@ -71,7 +71,8 @@ StagedOccupancy staged_occupancy(int dt, int col)
 }
 
 struct AuxLaunchers {
-    GroupLauncher gather, refd_velocity, refd_stress;
+    void (*gather)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* group_args);
+    GroupLauncher refd_velocity, refd_stress;
     void (*fill_eq)(const void*, double, double, double, double, cudaStream_t);
     void (*init_macro)(const void*, double, double, double, double, cudaStream_t);
     void (*output_fields)(const void*, const OutputParams&, const uint8_t*, float*, cudaStream_t);
@@ -526,41 +527,39 @@ bool can_stage(const nnlbm_ctx* ctx, const Group& g)
     return true;
 }
 
-// the step kernel's launch: the staged form runs persistent warps, as many blocks as stay
-// resident (or fewer, one warp per unit of work at most); the others one warp per unit
-struct StepShape {
-    dim3 grid, block;
-    int form;
-};
-StepShape step_shape(const Group& g)
-{
-    if (g.staged) {
-        const int per_block = kStagedThreads / kChunk;
-        const int blocks = std::max(1, std::min((step_warps(g) + per_block - 1) / per_block, g.staged_max_blocks));
-        return {dim3(blocks), dim3(kStagedThreads), FORM_STAGED};
-    }
-    const int per_block = g.block / kChunk;
-    return {dim3((step_warps(g) + per_block - 1) / per_block), dim3(g.block), g.paired ? FORM_PAIRED : FORM_ONE};
-}
-
-// enqueue one step of a group (no host synchronisation); `odd` is the A-A parity
-int enqueue_step(nnlbm_ctx* ctx, Group& g, bool odd)
+// the kernels of one step with the group arguments `args` (no host synchronisation); `odd` is
+// the A-A parity.  `chained`: each kernel as a programmatic dependent of the one before it;
+// `only_step`: without the kernels before the step kernel itself
+int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool odd, bool chained, bool only_step = false)
 {
     const AuxLaunchers& A = aux_launchers(g.dtype);
     const int per_block = g.block / kChunk;
-    const dim3 cblk(g.block);
-    const StepShape sh = step_shape(g);
-    const dim3 rgrid((std::max(g.n_chunks, 1) + per_block - 1) / per_block); // one warp per chunk
-    if (g.any_refd) {
-        A.refd_velocity(odd, rgrid, cblk, ctx->stream, g.args.data());
-        A.refd_stress(odd, rgrid, cblk, ctx->stream, g.args.data());
+    auto blocks = [](int warps, int per) { return dim3(std::max((warps + per - 1) / per, 1)); };
+    if (!only_step && g.any_refd) {
+        const dim3 rgrid = blocks(g.n_chunks, per_block); // one warp per chunk
+        A.refd_velocity(odd, rgrid, dim3(g.block), ctx->stream, args);
+        A.refd_stress(odd, rgrid, dim3(g.block), ctx->stream, args);
     }
-    if (g.n_gather > 0) A.gather(odd, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, g.args.data());
-    step_launcher(g.dtype, g.collision)(odd, g.n_gather > 0, sh.form, sh.grid, sh.block, ctx->stream, g.args.data());
+    if (!only_step && g.n_gather > 0) A.gather(odd, chained, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
+    dim3 grid = blocks(step_warps(g), per_block), block(g.block);
+    int form = g.paired ? FORM_PAIRED : FORM_ONE;
+    if (g.staged) {
+        // persistent warps, as many blocks as stay resident (or fewer, one warp per unit at most)
+        grid = dim3(std::min((int)blocks(step_warps(g), kStagedThreads / kChunk).x, g.staged_max_blocks));
+        block = dim3(kStagedThreads);
+        form = FORM_STAGED;
+    }
+    step_launcher(g.dtype, g.collision)(odd, chained, form, grid, block, ctx->stream, args);
     CK(cudaGetLastError());
     return NNLBM_OK;
 }
 
+// kChainSteps steps of either starting parity as one CUDA graph: inside it the kernels follow one
+// another programmatically at 1.1-1.4 us a kernel, where one graph or kernel launch per step puts
+// 2-4 us between two steps (measured with empty kernels of 148 and 1000 blocks).  Shorter calls,
+// and the steps left over, are launched one by one, chained too: a call of a few steps pays for
+// no capture
+constexpr int kChainSteps = 16;
 int ensure_graphs(nnlbm_ctx* ctx, Group& g)
 {
     if (g.graph[0] && g.graph[1] && g.graph_gen == g.gen) return NNLBM_OK;
@@ -568,7 +567,9 @@ int ensure_graphs(nnlbm_ctx* ctx, Group& g)
         if (g.graph[p]) { cudaGraphExecDestroy(g.graph[p]); g.graph[p] = nullptr; }
         cudaGraph_t gr = nullptr;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = enqueue_step(ctx, g, p == 1);
+        int rc = NNLBM_OK;
+        for (int k = 0; k < kChainSteps && rc == NNLBM_OK; ++k)
+            rc = launch_step_kernels(ctx, g, g.args.data(), ((p + k) & 1) != 0, true);
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &gr);
         if (rc != NNLBM_OK) { if (gr) cudaGraphDestroy(gr); return rc; }
         if (e != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
@@ -692,12 +693,18 @@ int run_group_steps(nnlbm_ctx* ctx, Group& g, int64_t n, int flags, bool use_gra
 {
     int rc = prepare_steps(ctx, g, n, flags, reset);
     if (rc) return rc;
+    use_graph = use_graph && n >= 2 * kChainSteps;
     if (use_graph && (rc = ensure_graphs(ctx, g)) != NNLBM_OK) return rc;
     const int64_t parity = ctx->cases[g.cases[0]].parity;
-    for (int64_t k = 0; k < n; ++k) {
+    for (int64_t k = 0; k < n;) {
         const int p = (int)((parity + k) & 1);
-        if (use_graph) CK(cudaGraphLaunch(g.graph[p], ctx->stream));
-        else if ((rc = enqueue_step(ctx, g, p == 1)) != NNLBM_OK) return rc;
+        if (use_graph && n - k >= kChainSteps) {
+            CK(cudaGraphLaunch(g.graph[p], ctx->stream));
+            k += kChainSteps;
+        } else {
+            if ((rc = launch_step_kernels(ctx, g, g.args.data(), p == 1, true)) != NNLBM_OK) return rc;
+            ++k;
+        }
     }
     finish_steps(ctx, g, n, flags);
     return NNLBM_OK;
@@ -1738,13 +1745,11 @@ int nnlbm_profile_step(nnlbm_ctx* ctx, int ic, int64_t n_steps, int flags, doubl
             mark(4);
         }
         if (g.n_gather > 0) {
-            A.gather(odd, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, g.args.data());
+            A.gather(odd, false, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, g.args.data());
             mark(0);
         }
-        const StepShape sh = step_shape(g);
-        step_launcher(g.dtype, g.collision)(odd, false, sh.form, sh.grid, sh.block, ctx->stream, g.args.data());
+        if ((rc = launch_step_kernels(ctx, g, g.args.data(), odd, false, true)) != NNLBM_OK) return rc;
         mark(1);
-        CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(ctx->stream));
     for (size_t i = 1; i < ev.size(); ++i) {
@@ -1817,22 +1822,9 @@ int nnlbm_step_noalloc(nnlbm_ctx* ctx, int64_t n_steps, int flags)
         alignas(64) char args[kGroupArgsBytes];
         if (f64) noalloc_args<double>(g, gi, scratch, args);
         else noalloc_args<float>(g, gi, scratch, args);
-        const AuxLaunchers& A = aux_launchers(g.dtype);
-        const int per_block = g.block / kChunk;
-        const dim3 cblk(g.block);
-        const StepShape sh = step_shape(g);
-        const dim3 rgrid((std::max(g.n_chunks, 1) + per_block - 1) / per_block); // one warp per chunk
         const int64_t parity = ctx->cases[g.cases[0]].parity;
-        for (int64_t k = 0; k < n_steps; ++k) {
-            const bool odd = ((parity + k) & 1) != 0;
-            if (g.any_refd) {
-                A.refd_velocity(odd, rgrid, cblk, ctx->stream, args);
-                A.refd_stress(odd, rgrid, cblk, ctx->stream, args);
-            }
-            if (g.n_gather > 0) A.gather(odd, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
-            step_launcher(g.dtype, g.collision)(odd, false, sh.form, sh.grid, sh.block, ctx->stream, args);
-        }
-        CK(cudaGetLastError());
+        for (int64_t k = 0; k < n_steps; ++k)
+            if ((rc = launch_step_kernels(ctx, g, args, ((parity + k) & 1) != 0, true)) != NNLBM_OK) return rc;
         finish_steps(ctx, g, n_steps, flags);
     }
     // the cursors into the status block, where nnlbm_step keeps them (same layout), so that the
