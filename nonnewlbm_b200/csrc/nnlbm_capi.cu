@@ -94,7 +94,7 @@ namespace {
 const int kStorageBytes[4] = {8, 4, 2, 2};
 const int kChunk = 32;
 // which open-plane node a cell finishes (per cell while the work list is built)
-enum : uint8_t { kServeXneg = 1, kServeXpos = 2, kServeXreq = 4, kServeYneg = 8, kServeYpos = 16 };
+enum : uint8_t { kServeXneg = 1, kServeXpos = 2, kServeXreq = 4, kServeYneg = 8, kServeYpos = 16, kServeXeq = 32 };
 // slack around the populations and after the labels: every kernel reads only cells of the
 // box, so nothing is read here; the slack keeps each allocation's start and end away from
 // the first and last 32-cell row
@@ -139,6 +139,7 @@ struct Case {
     std::vector<ChunkNodes> chunk_nodes; // the open-plane nodes each chunk serves
     std::vector<int32_t> self_cell;  // cells handled by their own thread, in cell order
     std::vector<int32_t> gather_self;// self indices of the gathered nodes
+    std::vector<int32_t> batch_self; // self indices of the nodes with a lane of their own in the step
     std::vector<double> self_prof;   // [n_self][3] prescribed velocity of INFLOW_EQ nodes
     int64_t n_fluid = 0, n_bc = 0, left_area = 0, right_area = 0, n_inflow_eq = 0;
     double ivc_flux = 0, svc_flux = 0, rho_left = 1, rho_right = 1, rho_eq = 1;
@@ -170,8 +171,8 @@ struct Group {
     ChunkNodes* d_chunk_nodes = nullptr;
     int n_chunks = 0;
     int4* d_gather = nullptr;
-    int2* d_nodes = nullptr;
-    int n_gather = 0;
+    int4* d_nodes = nullptr;
+    int n_gather = 0, n_nodes = 0;
     void* d_bc_prof = nullptr;
     void* d_bc_buf = nullptr;
     int64_t n_self = 0;
@@ -410,7 +411,7 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
     std::vector<Chunk> chunks;
     std::vector<ChunkNodes> chunk_nodes;
     std::vector<int4> gather;
-    std::vector<int2> nodes;
+    std::vector<int4> nodes;
     std::vector<CT> prof;
     int64_t self_off = 0;
     g.any_refd = false;
@@ -420,22 +421,30 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
         g.any_refd |= c.d.cy_mode == NNLBM_CY_REF_FD;
         for (Chunk ch : c.chunks) {
             ch.cflags = (int)j | (ch.cflags & ~CH_CASE_MASK);
+            if (ch.cflags & (CH_SRC | CH_ROW)) ch.nodes += (int)chunk_nodes.size();
             chunks.push_back(ch);
         }
-        chunk_nodes.insert(chunk_nodes.end(), c.chunk_nodes.begin(), c.chunk_nodes.end());
+        for (ChunkNodes cn : c.chunk_nodes) {
+            if (cn.has_eq()) {
+                const CT u[3] = {(CT)c.self_prof[3 * (size_t)cn.eq_self], (CT)c.self_prof[3 * (size_t)cn.eq_self + 1],
+                                 (CT)c.self_prof[3 * (size_t)cn.eq_self + 2]};
+                static_assert(sizeof u <= sizeof cn.prof, "a prescribed velocity in the node record");
+                memcpy(cn.prof, u, sizeof u);
+            }
+            chunk_nodes.push_back(cn);
+        }
         // a paired step kernel takes chunks two by two: an odd count gets an empty chunk
         // (no colliding lane), so that no pair mixes two cases and the list length is even
         if (pairs_chunks(g.dtype, g.collision) && (c.chunks.size() & 1)) {
             Chunk none = chunks.back();
             none.fluid = 0;
             none.periodic = 0;
-            none.cflags &= ~CH_SRC;
+            none.cflags &= ~(CH_SRC | CH_ROW);
             chunks.push_back(none);
-            chunk_nodes.push_back(ChunkNodes{});
         }
         for (int32_t k : c.gather_self)
             gather.push_back(make_int4(c.self_cell[k], (int)j, (int)(self_off + k), (int)c.label[c.self_cell[k]]));
-        for (int32_t cell : c.self_cell) nodes.push_back(make_int2(cell, (int)j));
+        for (int32_t k : c.batch_self) nodes.push_back(make_int4(c.self_cell[k], (int)j, (int)(self_off + k), 0));
         for (double v : c.self_prof) prof.push_back((CT)v);
         self_off += (int64_t)c.self_cell.size();
     }
@@ -455,8 +464,8 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
     CK(cudaMalloc((void**)&g.d_chunk_nodes, std::max<size_t>(chunk_nodes.size(), 1) * sizeof(ChunkNodes)));
     if (!chunk_nodes.empty())
         CK(cudaMemcpy(g.d_chunk_nodes, chunk_nodes.data(), chunk_nodes.size() * sizeof(ChunkNodes), cudaMemcpyHostToDevice));
-    CK(cudaMalloc((void**)&g.d_nodes, std::max<size_t>(nodes.size(), 1) * sizeof(int2)));
-    if (!nodes.empty()) CK(cudaMemcpy(g.d_nodes, nodes.data(), nodes.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CK(cudaMalloc((void**)&g.d_nodes, std::max<size_t>(nodes.size(), 1) * sizeof(int4)));
+    if (!nodes.empty()) CK(cudaMemcpy(g.d_nodes, nodes.data(), nodes.size() * sizeof(int4), cudaMemcpyHostToDevice));
     CK(cudaMalloc((void**)&g.d_gather, std::max<size_t>(gather.size(), 1) * sizeof(int4)));
     if (!gather.empty()) CK(cudaMemcpy(g.d_gather, gather.data(), gather.size() * sizeof(int4), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&g.d_bc_prof, std::max<size_t>(prof.size(), 1) * sizeof(CT)));
@@ -465,6 +474,7 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
     CK(cudaMemset(g.d_bc_buf, 0, std::max<int64_t>(self_off, 1) * 4 * sizeof(CT)));
     g.n_chunks = (int)chunks.size();
     g.n_gather = (int)gather.size();
+    g.n_nodes = (int)nodes.size();
     // room in L2 for the work lists the step launches mark persisting (the limit is this
     // process's; it is raised, never lowered, and capped by the device)
     {
@@ -492,7 +502,7 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
     ga.gather = g.d_gather;
     ga.n_gather = g.n_gather;
     ga.nodes = g.d_nodes;
-    ga.n_nodes = (int)g.n_self;
+    ga.n_nodes = g.n_nodes;
     ga.bc_prof = (const CT*)g.d_bc_prof;
     ga.bc_buf = (CT*)g.d_bc_buf;
     ga.cursor = g.d_ints;
@@ -514,7 +524,7 @@ int prepare_group(nnlbm_ctx* ctx, Group& g)
 int step_warps(const Group& g)
 {
     const int cw = g.paired ? g.n_chunks / 2 : g.n_chunks;
-    return std::max(cw + (int)((g.n_self + 31) / 32), 1);
+    return std::max(cw + (g.n_nodes + 31) / 32, 1);
 }
 
 // whether a group can step in the staged form: its collision pairs, the kernel fits on the
@@ -1049,10 +1059,33 @@ int nnlbm_set_map(nnlbm_ctx* ctx, int ic, const uint8_t* map)
                 continue;
             }
         }
+        // a GEO_INFLOW node takes nothing from its neighbour, but the warp of a colliding cell at
+        // x + 1 writes its slots with its own (one node a chunk)
+        if (can_fuse && lab == L_IN_EQ && (int)(i % nx) < nx - 1 && (map[i + 1] == L_FLUID || map[i + 1] == L_PERIODIC))
+            serves[i + 1] |= kServeXeq;
         dl[i] |= LF_SELF;
         if (lab != L_IN_EQ) gather_self.push_back((int32_t)self_cell.size());
         self_cell.push_back((int32_t)i);
     }
+    // The cells whose slots the gather of a step reads, and which the step must not overwrite
+    // before: within three cells of a gathered node on each axis (its stencil reaches two cells
+    // inward and one to the sides, a slot lies one cell from the population it holds), around the
+    // box like the A-A stores.  Without fused nodes every open-plane node is gathered, and every
+    // chunk waits.
+    std::vector<uint8_t> waits;
+    if (can_fuse && !gather_self.empty()) {
+        waits.assign((size_t)c.N, 0);
+        for (int32_t k : gather_self) {
+            const size_t i = (size_t)self_cell[k];
+            const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
+            auto around = [](int v, int n) { return ((v % n) + n) % n; };
+            for (int dz = -3; dz <= 3; ++dz)
+                for (int dy = -3; dy <= 3; ++dy)
+                    for (int dx = -3; dx <= 3; ++dx) waits[id(around(x + dx, nx), around(y + dy, ny), around(z + dz, nz))] = 1;
+        }
+    }
+    const bool all_wait = !can_fuse && !gather_self.empty();
+    std::vector<uint8_t> served_eq(self_cell.size(), 0);
     // halfway bounce-back: per cell, bit q where the neighbour x + c_q (wrapped) is a wall
     std::vector<uint32_t> hw;
     if (c.d.bounce_back == NNLBM_BB_HALFWAY) {
@@ -1097,7 +1130,15 @@ int nnlbm_set_map(nnlbm_ctx* ctx, int ic, const uint8_t* map)
                         if (serves[i] & kServeXreq) cn.xreq |= bit;
                         if (serves[i] & kServeYneg) cn.yneg |= bit;
                         if (serves[i] & kServeYpos) cn.ypos |= bit;
+                        if ((serves[i] & kServeXeq) && !cn.xeq) {
+                            const size_t k = std::lower_bound(self_cell.begin(), self_cell.end(), (int32_t)(i - 1)) - self_cell.begin();
+                            served_eq[k] = 1;
+                            cn.xneg |= bit;
+                            cn.xeq = bit;
+                            cn.eq_self = (unsigned)k;
+                        }
                         if (!hw.empty() && hw[i]) ch.cflags |= CH_HW;
+                        if (all_wait || (!waits.empty() && waits[i])) ch.cflags |= CH_WAIT;
                     }
                 }
                 // flags: the chunk lies on a y or z face; the chunk is plain (no colliding cell
@@ -1105,17 +1146,37 @@ int nnlbm_set_map(nnlbm_ctx* ctx, int ic, const uint8_t* map)
                 const bool face = y == 0 || y == ny - 1 || z == 0 || z == nz - 1;
                 const unsigned xface = (x0 == 0 ? 1u : 0u) | (nx - 1 - x0 < kChunk ? 1u << (nx - 1 - x0) : 0u);
                 const bool plain = !face && !(ch.fluid & xface) && !(ch.cflags & CH_HW);
+                // nodes of x planes that are lanes of a plain chunk leave with the row's own stores
+                // (a node has one inward cell; of two cells that would serve one lane, neither does)
+                const unsigned self = ~ch.fluid;
+                if (plain && hw.empty()) {
+                    cn.row_l = (cn.xneg >> 1) & self;
+                    cn.row_r = (cn.xpos << 1) & self & ~cn.row_l;
+                    cn.row_eq = (((cn.xeq >> 1) & cn.row_l) | ((cn.xreq << 1) & cn.row_r));
+                    cn.xneg &= ~(cn.row_l << 1);
+                    cn.xeq &= ~(cn.row_l << 1);
+                    cn.xpos &= ~(cn.row_r >> 1);
+                    cn.xreq &= ~(cn.row_r >> 1);
+                }
+                const bool rows = (cn.row_l | cn.row_r) != 0;
                 const bool serving = (cn.xneg | cn.xpos | cn.yneg | cn.ypos) != 0;
-                ch.cflags |= CH_FLUID | (face ? CH_FACE : 0) | (plain ? CH_PLAIN : 0) | (serving ? CH_SRC : 0);
+                ch.cflags |= CH_FLUID | (face ? CH_FACE : 0) | (plain ? CH_PLAIN : 0) | (serving ? CH_SRC : 0) | (rows ? CH_ROW : 0);
+                if (serving || rows) {
+                    ch.nodes = (int)chunk_nodes.size();
+                    chunk_nodes.push_back(cn);
+                }
                 chunks.push_back(ch);
-                chunk_nodes.push_back(cn);
             }
+    std::vector<int32_t> batch_self;
+    for (size_t k = 0; k < self_cell.size(); ++k)
+        if (!served_eq[k]) batch_self.push_back((int32_t)k);
     c.label.assign(map, map + c.N);
     c.dlabel = dl;
     c.chunks = chunks;
     c.chunk_nodes = chunk_nodes;
     c.self_cell = self_cell;
     c.gather_self = gather_self;
+    c.batch_self = batch_self;
     c.self_prof.assign(self_cell.size() * 3, 0.0);
     c.n_fluid = nfl; c.left_area = la; c.right_area = ra; c.n_inflow_eq = neq; c.n_bc = nbc;
     CK(cudaSetDevice(ctx->device));

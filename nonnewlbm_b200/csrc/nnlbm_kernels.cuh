@@ -147,20 +147,28 @@ __device__ __forceinline__ const void* odd_ld(const CaseArgs<CT>& a, int q)
 // one 32-cell row chunk of the work list: the first cell, its row, the case and flags,
 // and per lane (bit = lane) which cells collide and which of those are PERIODIC
 struct alignas(16) Chunk {
-    int c0, yz, cflags, pad0;
+    int c0, yz, cflags, nodes;
     unsigned fluid, periodic, pad1, pad2;
 };
-// per chunk (in a parallel array read only by serve_nodes): which lanes finish an open-plane
-// node next to them, the node at x-1 (IN_L), at x+1 (IN_R, or OUT_REQ where the lane is in
-// xreq too), at y-1 (OUT_F), at y+1 (OUT_B)
+// one per serving chunk (Chunk::nodes): which lanes finish an open-plane node next to them, the
+// node at x-1 (IN_L, or IN_EQ where the lane is in xeq too), at x+1 (IN_R, or OUT_REQ where the
+// lane is in xreq too), at y-1 (OUT_F), at y+1 (OUT_B).  Nodes of x planes that lie in the lanes of
+// a plain chunk themselves are in none of these: row_l has the node lanes whose inward cell is
+// lane + 1, row_r those whose inward cell is lane - 1, row_eq those of either that are IN_EQ or
+// OUT_REQ (else IN_L, IN_R).  prof: the prescribed velocity of the chunk's IN_EQ node (three
+// CT), at most one a chunk
 struct alignas(16) ChunkNodes {
-    unsigned xneg, xpos, xreq, yneg, ypos, pad0, pad1, pad2;
+    unsigned xneg, xpos, xreq, yneg, ypos, xeq, eq_self, row_l;
+    unsigned prof[6], row_r, row_eq;
+    __host__ bool has_eq() const { return xeq != 0 || (row_eq & row_l) != 0; }
 };
 // chunk flags (bits 16.. of cflags, the case index below).  CH_PLAIN: no neighbour of any
 // colliding lane wraps around the box (the chunk is off the y/z faces and has no
-// colliding cell at x = 0 or nx-1); CH_SRC: some lane finishes an open-plane node
+// colliding cell at x = 0 or nx-1); CH_SRC: some lane finishes an open-plane node; CH_WAIT: some
+// lane's slots are read by the gather of the same step; CH_ROW: some lanes that do not collide are
+// open-plane nodes finished in place (ChunkNodes::row_l, row_r)
 enum : int { CH_CASE_MASK = 0xffff, CH_FLUID = 1 << 16, CH_FACE = 1 << 17, CH_PLAIN = 1 << 18, CH_SRC = 1 << 19,
-             CH_HW = 1 << 20 };
+             CH_HW = 1 << 20, CH_WAIT = 1 << 21, CH_ROW = 1 << 22 };
 // bits of a case's watchdog word: a density out of range (or not finite), a bounded wait of
 // the staged step that gave up
 enum : int { ERR_DENSITY = 1, ERR_STALL = 2 };
@@ -180,13 +188,13 @@ struct GroupArgs {
     int n_cases, pad2;
     const CaseArgs<CT>* cases;
     const Chunk* chunks;
-    const ChunkNodes* chunk_nodes;  // [n_chunks]
+    const ChunkNodes* chunk_nodes;  // of the serving chunks
     int n_chunks, pad0;
     const int4* gather;        // {cell, case, node index, label} of the open-plane nodes
     int n_gather, n_nodes;
-    const int2* nodes;         // [n_nodes] {cell, case} of every boundary node (open planes, INFLOW_EQ)
-    const CT* bc_prof;         // [n_nodes][3] prescribed velocity (GEO_INFLOW nodes)
-    CT* bc_buf;                // [n_nodes][4] gathered rho, ux, uy, uz
+    const int4* nodes;         // [n_nodes] {cell, case, node index} of the boundary nodes with a lane of their own
+    const CT* bc_prof;         // [node index][3] prescribed velocity (GEO_INFLOW nodes)
+    CT* bc_buf;                // [node index][4] gathered rho, ux, uy, uz
     // step cursors into every case's ctl, one per A-A parity: a step of parity p reads
     // cursor[p] and stores cursor[p] + 1 into cursor[1 - p], which no kernel of the step
     // reads, so no launch needs a grid-wide count
@@ -218,7 +226,8 @@ __host__ __device__ constexpr int args_mode(int n_cases)
 // gather, where it has nodes to gather, and the step kernel.
 //   - The first kernel of a step waits for the step before as its first act.
 //   - The gather then lets the step kernel start at once.  The slots that it reads are
-//     overwritten by the step, whose warps wait for it before their first store.  The step kernel itself leaves the next kernel's start to
+//     overwritten by the step: the chunks that hold them (CH_WAIT) and the node warps wait for
+//     it before their first store.  The step kernel itself leaves the next kernel's start to
 //     its own end: with an earlier trigger the next step's blocks come up while this one's are
 //     running, and measured slower (pipe 96x32x32 7.5 us a step against 6.5, junction 31.2
 //     against 30.1).
@@ -343,16 +352,22 @@ __device__ __forceinline__ double node_outputs(const CaseArgs<CT>& a, int flags,
 // chunk's cells have stored, the node's equilibrium goes into the node's slots (which no
 // other cell touches within the step) with the node's outputs, and no separate gather, with
 // its wait before the first store, is needed.  The chunk's lane masks say which nodes its
-// lanes finish.  Where few lanes serve (an inlet row has one), the whole warp writes each
-// node, lane q storing population q; where many serve (an outlet row), each lane writes its
-// own.
-
-// the chunks that serve nodes are few; their node code stays out of line unless the build
-// asks otherwise
-#ifndef NNLBM_SERVE_INLINE
-#define NNLBM_SERVE_INLINE __noinline__
-#endif
-
+// lanes finish.  Where few lanes serve (a row of an inlet or outlet plane across x has one), the whole warp
+// writes each node, lane q storing population q; where many serve (an outlet row), each lane
+// writes its own.
+//
+// A GEO_INFLOW node with a colliding cell at x + 1 is written the same way by that cell's warp:
+// it takes nothing from the cell, but its slots lie in the sectors that the warp writes anyway.
+//
+// Where the node of an x plane is a lane of the chunk itself (the first or last cell of a row of
+// a box), that lane takes the state from the lane beside it, and its 27 values leave with the
+// row's own stores (row_nodes): no store of its own, and whole sectors.  Written by the warp
+// one by one after the others, as 27 requests of one element, such nodes took 53 of 343 us
+// of a step of an FP32 box of 256x192x160 cells with an inlet and an outlet plane, and 150 of 920
+// us with FP16 storage at 384x288x240.
+//
+// The node records are loaded with the populations (NodeWords), so that no load is left for
+// after the collision.
 // the node of serving lane direction d (0: x-1, 1: x+1, 2: y-1, 3: y+1) and its label
 __device__ __forceinline__ int served_label(int d, bool req)
 {
@@ -393,66 +408,165 @@ __device__ __forceinline__ void served_outputs(const CaseArgs<CT>& a, int flags,
     }
 }
 
-// called by the whole warp of a chunk with serving lanes (CH_SRC), after its stores; rho and
-// u are each lane's pre-collision values
+// a serving chunk's node record, a word a lane (words of ChunkNodes in order)
+struct NodeWords {
+    unsigned w;
+    __device__ __forceinline__ unsigned get(int k) const { return __shfl_sync(0xffffffffu, w, k); }
+    __device__ __forceinline__ void prof(int k, float& v) const { v = __uint_as_float(get(8 + k)); }
+    __device__ __forceinline__ void prof(int k, double& v) const
+    {
+        const unsigned lo = get(8 + 2 * k), hi = get(9 + 2 * k);
+        v = __hiloint2double((int)hi, (int)lo);
+    }
+};
+
+// the equilibrium of kind `eq` other than the factorised one, as stored values (out of line)
+template <int DT>
+__device__ __noinline__ void stored_equilibrium(int eq, typename Storage<DT>::CT scale, typename Storage<DT>::CT r,
+                                                typename Storage<DT>::CT u, typename Storage<DT>::CT v, typename Storage<DT>::CT w,
+                                                typename Storage<DT>::CT* f)
+{
+    using CT = typename Storage<DT>::CT;
+#pragma unroll 1
+    for (int q = 0; q < 27; ++q) {
+        const CT fq = feq_one<CT>(eq, q, r, u, v, w);
+        f[q] = DT == 0 ? fq : DT == 1 ? fq - weight<CT>(q) : mad(fq, scale, -(weight<CT>(q) * scale));
+    }
+}
+
+// the open-plane nodes among the lanes of a chunk (CH_ROW), called by the whole warp between the
+// collision and the stores: rho, u are each lane's pre-collision values, f the values it stores.
+// Returns whether this lane is such a node, with f its equilibrium
 template <int DT, bool ODD>
-__device__ NNLBM_SERVE_INLINE void serve_nodes(const CaseArgs<typename Storage<DT>::CT>* ap, const Chunk* chp,
-                                               const ChunkNodes* cnp, int lane, typename Storage<DT>::CT rho,
-                                               typename Storage<DT>::CT ux, typename Storage<DT>::CT uy,
-                                               typename Storage<DT>::CT uz, int step, int flags)
+__device__ __forceinline__ bool row_nodes(const CaseArgs<typename Storage<DT>::CT>& a, const NodeWords& nw, int lane, int c, int step,
+                                          int flags, typename Storage<DT>::CT rho, typename Storage<DT>::CT ux,
+                                          typename Storage<DT>::CT uy, typename Storage<DT>::CT uz, typename Storage<DT>::CT* f)
+{
+    using CT = typename Storage<DT>::CT;
+    const unsigned l = nw.get(7), r = nw.get(14), eq = nw.get(15), bit = 1u << lane;
+    const int in = lane + ((l & bit) ? 1 : 0) - ((r & bit) ? 1 : 0);
+    const CT ri = __shfl_sync(0xffffffffu, rho, in), ui = __shfl_sync(0xffffffffu, ux, in);
+    const CT vi = __shfl_sync(0xffffffffu, uy, in), wi = __shfl_sync(0xffffffffu, uz, in);
+    CT p0, p1, p2;
+    nw.prof(0, p0); nw.prof(1, p1); nw.prof(2, p2);
+    if (!((l | r) & bit)) return false;
+    const StepCtl<CT>& ctl = a.ctl[step];
+    const int lab = (l & bit) ? ((eq & bit) ? (int)L_IN_EQ : (int)L_IN_L) : ((eq & bit) ? (int)L_OUT_REQ : (int)L_IN_R);
+    CT rn, u, v, w;
+    if (lab == L_IN_EQ) { // lbm_bc.h:126-129
+        rn = ctl.rho_eq; u = p0 * ctl.prof_scale; v = p1 * ctl.prof_scale; w = p2 * ctl.prof_scale;
+    } else {
+        served_state<CT>(lab, ri, ui, vi, wi, ctl, rn, u, v, w);
+    }
+    if (a.eq <= EQ_INV_CUM) {
+        // feq_one's factorised equilibrium, factor by factor
+        const CT X[3] = {inv_cum_factor<CT>(-1, u), inv_cum_factor<CT>(0, u), inv_cum_factor<CT>(1, u)};
+        const CT Y[3] = {inv_cum_factor<CT>(-1, v), inv_cum_factor<CT>(0, v), inv_cum_factor<CT>(1, v)};
+        const CT Z[3] = {inv_cum_factor<CT>(-1, w), inv_cum_factor<CT>(0, w), inv_cum_factor<CT>(1, w)};
+#pragma unroll
+        for (int q = 0; q < 27; ++q) {
+            const int n = nnzq(q);
+            const CT pre = n == 0 ? CT(-1.0 / 27.0) : n == 1 ? CT(1.0 / 54.0) : n == 2 ? CT(-1.0 / 108.0) : CT(1.0 / 216.0);
+            CT fq = pre * rn * (X[q / 9] * Y[(q / 3) % 3] * Z[q % 3]);
+            if (q == 18 && a.eq == EQ_INV_CUM_REF) fq *= rn; // the shipped feq_pmm (lbm_eq_inv_cum.h:49)
+            f[q] = DT == 0 ? fq : DT == 1 ? fq - weight<CT>(q) : mad(fq, a.scale, -(weight<CT>(q) * a.scale));
+        }
+    } else {
+        CT t[27];
+        stored_equilibrium<DT>(a.eq, a.scale, rn, u, v, w, t);
+#pragma unroll
+        for (int q = 0; q < 27; ++q) f[q] = t[q];
+    }
+    served_outputs<CT>(a, flags, lab, c, rn, u, v, w);
+    return true;
+}
+
+// many serving lanes: each writes its own nodes (out of line: outlet rows only)
+template <int DT, bool ODD>
+__device__ __noinline__ void serve_rows(const CaseArgs<typename Storage<DT>::CT>* ap, int c, int x, int y, int z, unsigned dirs,
+                                        bool req, typename Storage<DT>::CT rho, typename Storage<DT>::CT ux,
+                                        typename Storage<DT>::CT uy, typename Storage<DT>::CT uz, int step, int flags)
 {
     using S = Storage<DT>;
     using T = typename S::T;
     using CT = typename S::CT;
     const CaseArgs<CT>& a = *ap;
-    // the records are read here rather than kept in registers through the collision
-    const int c0 = chp->c0, yz = chp->yz;
-    const unsigned xneg = cnp->xneg, xpos = cnp->xpos, xreq = cnp->xreq, yneg = cnp->yneg, ypos = cnp->ypos;
+    const int sy = a.nx;
+    const StepCtl<CT>& ctl = a.ctl[step];
+    for (int d = 0; d < 4; ++d) {
+        if (!((dirs >> d) & 1u)) continue;
+        const int lab = served_label(d, req);
+        const int xn = x - (d == 0) + (d == 1), yn = y - (d == 2) + (d == 3);
+        const int n = c + (d == 0 ? -1 : d == 1 ? 1 : d == 2 ? -sy : sy);
+        CT r, u, v, w;
+        served_state<CT>(lab, rho, ux, uy, uz, ctl, r, u, v, w);
+        CT f[27];
+        equilibrium<CT>(a.eq, r, u, v, w, f);
+        const uint32_t hwm = (ODD && a.hw) ? a.hw[n] : 0u; // halfway: populations headed into a wall stay
+#pragma unroll
+        for (int q = 0; q < 27; ++q) {
+            if (!ODD || ((hwm >> q) & 1u)) S::store((T*)a.slot_even[oppq(q)], n, q, f[q], a.scale);
+            else S::store((T*)a.slot_odd_st[q], n + node_wrap(xn, yn, z, q, a.nx, a.ny, a.nz), q, f[q], a.scale);
+        }
+        served_outputs<CT>(a, flags, lab, n, r, u, v, w);
+    }
+}
+
+// called by the whole warp of a chunk with serving lanes (CH_SRC), after its stores; `word` is
+// each lane's word of the node record, rho and u its pre-collision values.  Out of line: inlined
+// it costs the bulk path 7 registers, and with 80 spills
+template <int DT, bool ODD>
+__device__ __noinline__ void serve_nodes(const CaseArgs<typename Storage<DT>::CT>* ap, const Chunk* chp, unsigned word,
+                                         typename Storage<DT>::CT rho, typename Storage<DT>::CT ux, typename Storage<DT>::CT uy,
+                                         typename Storage<DT>::CT uz, int step, int flags)
+{
+    using S = Storage<DT>;
+    using T = typename S::T;
+    using CT = typename S::CT;
+    const CaseArgs<CT>& a = *ap;
+    const NodeWords nw{word};
+    const int lane = threadIdx.x & 31, c0 = chp->c0, yz = chp->yz;
+    const unsigned xneg = nw.get(0), xpos = nw.get(1), xreq = nw.get(2), yneg = nw.get(3), ypos = nw.get(4), xeq = nw.get(5);
     const int y = yz & 0xffff, z = yz >> 16;
     const int sy = a.nx, x0 = c0 - y * sy - z * sy * a.ny;
-    const StepCtl<CT>& ctl = a.ctl[step];
-    const unsigned masks[4] = {xneg, xpos, yneg, ypos};
-    const unsigned src = xneg | xpos | yneg | ypos;
-    if (__popc(src) > 4) {
-        // many serving lanes: each writes its own nodes
+    unsigned few = xneg | xpos | yneg | ypos;
+    if (__popc(few & ~xeq) > 4) {
         const unsigned bit = 1u << lane;
-        for (int d = 0; d < 4; ++d) {
-            if (!(masks[d] & bit)) continue;
-            const int lab = served_label(d, (xreq & bit) != 0);
-            const int xn = x0 + lane - (d == 0) + (d == 1), yn = y - (d == 2) + (d == 3);
-            const int n = c0 + lane + (d == 0 ? -1 : d == 1 ? 1 : d == 2 ? -sy : sy);
-            CT r, u, v, w;
-            served_state<CT>(lab, rho, ux, uy, uz, ctl, r, u, v, w);
-            CT f[27];
-            equilibrium<CT>(a.eq, r, u, v, w, f);
-            const uint32_t hwm = (ODD && a.hw) ? a.hw[n] : 0u; // halfway: populations headed into a wall stay
-#pragma unroll
-            for (int q = 0; q < 27; ++q) {
-                if (!ODD || ((hwm >> q) & 1u)) S::store((T*)a.slot_even[oppq(q)], n, q, f[q], a.scale);
-                else S::store((T*)a.slot_odd_st[q], n + node_wrap(xn, yn, z, q, a.nx, a.ny, a.nz), q, f[q], a.scale);
-            }
-            served_outputs<CT>(a, flags, lab, n, r, u, v, w);
-        }
-        return;
+        const unsigned dirs = ((xneg & ~xeq & bit) ? 1u : 0u) | ((xpos & bit) ? 2u : 0u) | ((yneg & bit) ? 4u : 0u) |
+                              ((ypos & bit) ? 8u : 0u);
+        if (dirs) serve_rows<DT, ODD>(ap, c0 + lane, x0 + lane, y, z, dirs, (xreq & bit) != 0, rho, ux, uy, uz, step, flags);
+        few = xeq; // the GEO_INFLOW node is left, which the whole warp writes
     }
     // few serving lanes: the warp writes each node, lane q population q
-    for (unsigned todo = src; todo; todo &= todo - 1) {
+    const bool rows = few == xeq;
+    for (unsigned todo = few; todo; todo &= todo - 1) {
         const int s = __ffs(todo) - 1;
         const CT rs = __shfl_sync(0xffffffffu, rho, s), us = __shfl_sync(0xffffffffu, ux, s);
         const CT vs = __shfl_sync(0xffffffffu, uy, s), ws = __shfl_sync(0xffffffffu, uz, s);
+        CT p0, p1, p2;
+        nw.prof(0, p0); nw.prof(1, p1); nw.prof(2, p2);
         for (int d = 0; d < 4; ++d) {
-            if (!((masks[d] >> s) & 1u)) continue;
-            const int lab = served_label(d, ((xreq >> s) & 1u) != 0);
+            const unsigned m = d == 0 ? xneg : d == 1 ? xpos : d == 2 ? yneg : ypos;
+            const bool eq = d == 0 && ((xeq >> s) & 1u);
+            if (!((m >> s) & 1u) || (rows && !eq)) continue;
+            const int lab = eq ? (int)L_IN_EQ : served_label(d, ((xreq >> s) & 1u) != 0);
             const int xn = x0 + s - (d == 0) + (d == 1), yn = y - (d == 2) + (d == 3);
             const int n = c0 + s + (d == 0 ? -1 : d == 1 ? 1 : d == 2 ? -sy : sy);
+            const StepCtl<CT>& ctl = a.ctl[step];
             CT r, u, v, w;
-            served_state<CT>(lab, rs, us, vs, ws, ctl, r, u, v, w);
+            if (eq) { // lbm_bc.h:126-129
+                r = ctl.rho_eq; u = p0 * ctl.prof_scale; v = p1 * ctl.prof_scale; w = p2 * ctl.prof_scale;
+            } else {
+                served_state<CT>(lab, rs, us, vs, ws, ctl, r, u, v, w);
+            }
             if (lane < 27) {
                 const int q = lane;
                 const CT fq = feq_one<CT>(a.eq, q, r, u, v, w);
                 const bool stay = ODD && a.hw && ((a.hw[n] >> q) & 1u); // halfway: headed into a wall
-                if (!ODD || stay) S::store((T*)a.slot_even[oppq(q)], n, q, fq, a.scale);
-                else S::store((T*)a.slot_odd_st[q], n + node_wrap(xn, yn, z, q, a.nx, a.ny, a.nz), q, fq, a.scale);
+                T* const df = (T*)a.df;
+                if (!ODD || stay) S::store(df, (int64_t)oppq(q) * a.qstride + n, q, fq, a.scale);
+                else S::store(df, (int64_t)q * a.qstride + n + cxq(q) + sy * (cyq(q) + (int64_t)a.ny * czq(q)) +
+                              node_wrap(xn, yn, z, q, a.nx, a.ny, a.nz), q, fq, a.scale);
             }
             if (lane == s) served_outputs<CT>(a, flags, lab, n, r, u, v, w);
         }
@@ -543,85 +657,144 @@ struct StepRegs {
 // pointer plus an offset made of the slot, row and plane strides only; the rare chunks on
 // a face wrap their neighbour indices around the box.
 // ---------------------------------------------------------------------------------------
+// Chunks next to a face or (halfway bounce-back) to a wall, odd step: a cell's 27 accesses with
+// the neighbour indices wrapped around the box, and with the bits of hwm for directions whose
+// neighbour is a wall.  For 16-bit storage out of line on a copy, so that the plain path has its
+// registers to itself (a box of FP16 cells between walls, 26.5 M: 780 us against 805 inline);
+// in line with FP32 and FP64 (FP32, 7.9 M cells: 289 us against 308 out of line; halfway
+// junction x0.6, MRT_LES: 15.8 against 16.5)
+template <int DT>
+__device__ __forceinline__ void general_load(const CaseArgs<typename Storage<DT>::CT>& a, int c, int yz, uint32_t hwm,
+                                             typename Storage<DT>::CT* f)
+{
+    using S = Storage<DT>;
+    using T = typename S::T;
+    const int y = yz & 0xffff, z = yz >> 16, x = c - a.nx * (y + z * a.ny);
+    const int64_t sy = a.nx, sz = (int64_t)a.nx * a.ny;
+    const T* p = (const T*)a.df;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int64_t n = wrapc(x - cxq(q), a.nx) + sy * wrapc(y - cyq(q), a.ny) + sz * wrapc(z - czq(q), a.nz);
+        f[q] = S::raw(((hwm >> oppq(q)) & 1u) ? p[q * a.qstride + c] : p[oppq(q) * a.qstride + n]);
+    }
+}
+template <int DT>
+__device__ __forceinline__ void general_store(const CaseArgs<typename Storage<DT>::CT>& a, int c, int yz, uint32_t hwm,
+                                              const typename Storage<DT>::CT* f)
+{
+    using S = Storage<DT>;
+    using T = typename S::T;
+    const int y = yz & 0xffff, z = yz >> 16, x = c - a.nx * (y + z * a.ny);
+    const int64_t sy = a.nx, sz = (int64_t)a.nx * a.ny;
+    T* p = (T*)a.df;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int64_t n = wrapc(x + cxq(q), a.nx) + sy * wrapc(y + cyq(q), a.ny) + sz * wrapc(z + czq(q), a.nz);
+        p[((hwm >> q) & 1u) ? oppq(q) * a.qstride + c : q * a.qstride + n] = S::put(f[q]);
+    }
+}
+template <int DT>
+__device__ __noinline__ void general_load_call(const CaseArgs<typename Storage<DT>::CT>* ap, int c, int yz, uint32_t hwm,
+                                               typename Storage<DT>::CT* f)
+{
+    general_load<DT>(*ap, c, yz, hwm, f);
+}
+template <int DT>
+__device__ __noinline__ void general_store_call(const CaseArgs<typename Storage<DT>::CT>* ap, int c, int yz, uint32_t hwm,
+                                                const typename Storage<DT>::CT* f)
+{
+    general_store<DT>(*ap, c, yz, hwm, f);
+}
+
 template <int DT, int COL, bool ODD>
 __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>::CT>& a, const CaseArgs<typename Storage<DT>::CT>* ap,
-                                            const Chunk& ch, const Chunk* chp, const ChunkNodes* cnp, int step, int flags,
+                                            const Chunk& ch, const Chunk* chp, const ChunkNodes* nodes, int step, int flags,
                                             int lane)
 {
     using S = Storage<DT>;
     using T = typename S::T;
     using CT = typename S::CT;
-    double mass = 0.0;
     const unsigned bit = 1u << lane;
+    const bool on = (ch.fluid & bit) != 0;
+    const int c = ch.c0 + lane;
+    // the even step touches the cell's own slots only; the odd step's general path wraps
+    const bool general = ODD && !(ch.cflags & CH_PLAIN);
     CT rho = CT(1), ux = CT(0), uy = CT(0), uz = CT(0);
-    if (ch.fluid & bit) {
-        const int c = ch.c0 + lane;
-        const int64_t qs = a.qstride, sy = a.nx, sz = (int64_t)a.nx * a.ny;
-        const bool plain = (ch.cflags & CH_PLAIN) != 0;
-        // the wrapped neighbour cell x + sign c_q of a face chunk
-        auto nbr = [&](int q, int sign) -> int64_t {
-            const int y = ch.yz & 0xffff, z = ch.yz >> 16;
-            const int x = ch.c0 - y * a.nx - z * a.nx * a.ny + lane;
-            return (int64_t)wrapc(x + sign * cxq(q), a.nx) + sy * wrapc(y + sign * cyq(q), a.ny) +
-                   sz * wrapc(z + sign * czq(q), a.nz) - c;
-        };
-        const T* pc = (const T*)a.df + c;
-        // halfway bounce-back: which neighbours are walls (CH_HW chunks, odd step only)
-        const uint32_t hwm = (ODD && (ch.cflags & CH_HW)) ? a.hw[c] : 0u;
-        CT f[27]; // the stored values
-        if (!ODD) {
-            // slot q at c
+    NodeWords nw{0u};
+    if (ch.cflags & (CH_SRC | CH_ROW)) nw.w = ((const unsigned*)(nodes + ch.nodes))[lane & 15];
+    CT f[27]; // the stored values
+    if (on) {
+        if (general && DT < 2) {
+            general_load<DT>(a, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, f);
+        } else if (general) {
+            CT t[27];
+            general_load_call<DT>(ap, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, t);
 #pragma unroll
-            for (int q = 0; q < 27; ++q) f[q] = S::raw(((const T*)a.slot_even[q])[c]);
-        } else if (plain) {
-            // slot opp(q) at c - c_q
-#pragma unroll
-            for (int q = 0; q < 27; ++q) f[q] = S::raw(((const T*)odd_ld(a, q))[c]);
+            for (int q = 0; q < 27; ++q) f[q] = t[q];
         } else {
+            // slot q at c, or slot opp(q) at c - c_q
 #pragma unroll
-            for (int q = 0; q < 27; ++q) f[q] = S::raw(((hwm >> oppq(q)) & 1u) ? pc[q * qs] : pc[oppq(q) * qs + nbr(q, -1)]);
+            for (int q = 0; q < 27; ++q) f[q] = S::raw(((const T*)(ODD ? odd_ld(a, q) : a.slot_even[q]))[c]);
         }
         CT fx = a.fx, fy = a.fy, fz = a.fz;
         if (a.cy_mode == CY_REF_FD && !(ch.periodic & bit)) {
             CT F[3] = {fx, fy, fz};
-            refd_force<CT>(ap, c, (int)sy, (int)sz, F);
+            refd_force<CT>(ap, c, a.nx, a.nx * a.ny, F);
             fx = F[0]; fy = F[1]; fz = F[2];
         }
         // one inlined collision for both viscosity models (the local Carreau-Yasuda law is
         // a runtime branch inside it)
-        CT Sl[6];
         const CYParams<CT> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
         step_cell<CT, COL, DT, DT != 0, CT>(f, fx, fy, fz, a.nu, a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, a.scale, a.inv_scale,
-                                            Sl, rho, ux, uy, uz);
-        // the gather of this step reads the slots written below
-        pdl_wait();
-        T* ps = (T*)a.df + c;
-        if (!ODD) {
-            // slot opp(q) at c
+                                            [&](CT r, CT u, CT v, CT w, const CT* Sl) {
+            rho = r; ux = u; uy = v; uz = w;
+            if ((flags & F_MACRO) || a.cy_mode == CY_REF_FD) {
+                write_macro<CT>(a, c, r, u, v, w, fx, fy, fz);
+                if (Sl) {
 #pragma unroll
-            for (int q = 0; q < 27; ++q) ((T*)a.slot_even[oppq(q)])[c] = S::put(f[q]);
-        } else if (plain) {
-            // slot q at c + c_q
-#pragma unroll
-            for (int q = 0; q < 27; ++q) ((T*)a.slot_odd_st[q])[c] = S::put(f[q]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 27; ++q) ps[((hwm >> q) & 1u) ? oppq(q) * qs : q * qs + nbr(q, 1)] = S::put(f[q]);
-        }
-        if ((flags & F_MACRO) || a.cy_mode == CY_REF_FD) {
-            write_macro<CT>(a, c, rho, ux, uy, uz, fx, fy, fz);
-            if (a.cy_mode == CY_LOCAL_NEQ) {
-#pragma unroll
-                for (int k = 0; k < 6; ++k) a.macro[(int64_t)(M_S11 + k) * a.N + c] = Sl[k];
+                    for (int k = 0; k < 6; ++k) a.macro[(int64_t)(M_S11 + k) * a.N + c] = Sl[k];
+                }
+            }
+            if (flags & F_STATS) accumulate_stats<CT>(a, c, r, u, v, w);
+            if (!(r > CT(0.25) && r < CT(4))) atomicOr(a.err, ERR_DENSITY);
+        });
+    }
+    bool put = on;
+    // the cell that the odd step's stores of c_x = -1 and c_x = +1 start from: a node of an x
+    // face wraps around the row
+    int cm = c, cp = c;
+    if (ch.cflags & CH_ROW) {
+        if (row_nodes<DT, ODD>(a, nw, lane, c, step, flags, rho, ux, uy, uz, f)) {
+            put = true;
+            if (ODD) {
+                const int x = c % a.nx;
+                if (x == 0) cm = c + a.nx;
+                if (x == a.nx - 1) cp = c - a.nx;
             }
         }
-        if (flags & F_STATS) accumulate_stats<CT>(a, c, rho, ux, uy, uz);
-        if (!(rho > CT(0.25) && rho < CT(4))) atomicOr(a.err, ERR_DENSITY);
-        mass = (double)rho;
     }
-    if (ch.cflags & CH_SRC) serve_nodes<DT, ODD>(ap, chp, cnp, lane, rho, ux, uy, uz, step, flags);
+    if (put) {
+        // the gather of this step reads the slots written below
+        if (ch.cflags & CH_WAIT) pdl_wait();
+        if (general && DT < 2) {
+            general_store<DT>(a, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, f);
+        } else if (general) {
+            CT t[27];
+#pragma unroll
+            for (int q = 0; q < 27; ++q) t[q] = f[q];
+            general_store_call<DT>(ap, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, t);
+        } else {
+            // slot opp(q) at c, or slot q at c + c_q
+#pragma unroll
+            for (int q = 0; q < 27; ++q) {
+                const int d = !ODD ? c : cxq(q) < 0 ? cm : cxq(q) > 0 ? cp : c;
+                ((T*)(ODD ? a.slot_odd_st[q] : a.slot_even[oppq(q)]))[d] = S::put(f[q]);
+            }
+        }
+    }
+    if (ch.cflags & CH_SRC) serve_nodes<DT, ODD>(ap, chp, nw.w, rho, ux, uy, uz, step, flags);
     if (flags & F_REDUCE) {
-        const double s0 = warp_sum(mass);
+        const double s0 = warp_sum(on ? (double)rho : 0.0);
         if (lane == 0 && s0 != 0.0) atomicAdd(red_stripe(a.red, global_warp()), s0);
     }
 }
@@ -806,8 +979,8 @@ __device__ __forceinline__ void pair_load_adjacent(const CaseArgs<float>& a, int
 // `adj`: an x-adjacent span (lane l holds cells c0 + 2l and c0 + 2l + 1)
 template <int DT, int COL, bool ODD>
 __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const CaseArgs<float>* ap, const Chunk& ca,
-                                            const Chunk& cb, const Chunk* cap, const ChunkNodes* cnp, f2* f, int step, int flags,
-                                            int lane, bool adj)
+                                            const Chunk& cb, const Chunk* cap, const ChunkNodes* nodes, f2* f, int step,
+                                            int flags, int lane, bool adj)
 {
     using T = typename Storage<DT>::T;
     const unsigned bit = 1u << lane;
@@ -817,13 +990,30 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
     if (fa || fb) {
         const int cA = adj ? ca.c0 + 2 * lane : ca.c0 + lane, cB = adj ? ca.c0 + 2 * lane + 1 : cb.c0 + lane;
         const f2 fx(a.fx), fy(a.fy), fz(a.fz);
-        f2 rho, ux, uy, uz;
-        f2 Sl[6];
         const CYParams<float> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
         step_cell<f2, COL, DT, false, float>(f, fx, fy, fz, f2(a.nu), a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, f2(a.scale),
-                                             f2(a.inv_scale), Sl, rho, ux, uy, uz);
+                                             f2(a.inv_scale), [&](f2 rho, f2 ux, f2 uy, f2 uz, const f2* Sl) {
+            r[0] = rho.v.x; r[1] = rho.v.y; u0[0] = ux.v.x; u0[1] = ux.v.y;
+            u1[0] = uy.v.x; u1[1] = uy.v.y; u2[0] = uz.v.x; u2[1] = uz.v.y;
+            const bool on[2] = {fa, fb};
+            const int cc[2] = {cA, cB};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (!on[h]) continue;
+                if (flags & F_MACRO) {
+                    write_macro<float>(a, cc[h], r[h], u0[h], u1[h], u2[h], a.fx, a.fy, a.fz);
+                    if (Sl) {
+#pragma unroll
+                        for (int k = 0; k < 6; ++k) a.macro[(int64_t)(M_S11 + k) * a.N + cc[h]] = h ? Sl[k].v.y : Sl[k].v.x;
+                    }
+                }
+                if (flags & F_STATS) accumulate_stats<float>(a, cc[h], r[h], u0[h], u1[h], u2[h]);
+                if (!(r[h] > 0.25f && r[h] < 4.f)) atomicOr(a.err, ERR_DENSITY);
+                mass += (double)r[h];
+            }
+        });
         // the gather of this step reads the slots written below
-        pdl_wait();
+        if ((ca.cflags | cb.cflags) & CH_WAIT) pdl_wait();
 #pragma unroll
         for (int q = 0; q < 27; ++q) {
             T* p = (T*)(ODD ? a.slot_odd_st[q] : a.slot_even[oppq(q)]);
@@ -835,28 +1025,12 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
                 pair_put<DT>(p + cB, v.v.y, fb);
             }
         }
-        r[0] = rho.v.x; r[1] = rho.v.y; u0[0] = ux.v.x; u0[1] = ux.v.y;
-        u1[0] = uy.v.x; u1[1] = uy.v.y; u2[0] = uz.v.x; u2[1] = uz.v.y;
-        const bool on[2] = {fa, fb};
-        const int cc[2] = {cA, cB};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (!on[h]) continue;
-            if (flags & F_MACRO) {
-                write_macro<float>(a, cc[h], r[h], u0[h], u1[h], u2[h], a.fx, a.fy, a.fz);
-                if (a.cy_mode == CY_LOCAL_NEQ) {
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) a.macro[(int64_t)(M_S11 + k) * a.N + cc[h]] = h ? Sl[k].v.y : Sl[k].v.x;
-                }
-            }
-            if (flags & F_STATS) accumulate_stats<float>(a, cc[h], r[h], u0[h], u1[h], u2[h]);
-            if (!(r[h] > 0.25f && r[h] < 4.f)) atomicOr(a.err, ERR_DENSITY);
-            mass += (double)r[h];
-        }
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        if ((h ? cb : ca).cflags & CH_SRC) serve_nodes<DT, ODD>(ap, cap + h, cnp + h, lane, r[h], u0[h], u1[h], u2[h], step, flags);
+        const Chunk& ch = h ? cb : ca;
+        if (!(ch.cflags & CH_SRC)) continue;
+        serve_nodes<DT, ODD>(ap, cap + h, ((const unsigned*)(nodes + ch.nodes))[lane & 15], r[h], u0[h], u1[h], u2[h], step, flags);
     }
     if (flags & F_REDUCE) {
         const double s0 = warp_sum(mass);
@@ -885,7 +1059,7 @@ template <int ARGS>
 __device__ __forceinline__ bool pairable(const GroupArgs<float>& g, const Chunk& ca, const Chunk& cb)
 {
     const int ci = ca.cflags & CH_CASE_MASK;
-    return ((ca.cflags & cb.cflags) & CH_PLAIN) && ci == (cb.cflags & CH_CASE_MASK) &&
+    return ((ca.cflags & cb.cflags) & CH_PLAIN) && !((ca.cflags | cb.cflags) & CH_ROW) && ci == (cb.cflags & CH_CASE_MASK) &&
            case_args<ARGS>(g, ci).cy_mode != CY_REF_FD;
 }
 
@@ -893,16 +1067,16 @@ __device__ __forceinline__ bool pairable(const GroupArgs<float>& g, const Chunk&
 // the equilibrium of its gathered (rho, u) (or of its prescribed inflow) into its own
 // slots, which no other cell reads or writes within the step, and adds its plane flux
 template <int DT, bool ODD>
-__device__ __noinline__ void node_batch(const int2* nodes, int n_nodes, const CaseArgs<typename Storage<DT>::CT>* cases,
-                                        const typename Storage<DT>::CT* bc_prof, const typename Storage<DT>::CT* bc_buf, int k,
+__device__ __noinline__ void node_batch(const int4* nodes, int n_nodes, const CaseArgs<typename Storage<DT>::CT>* cases,
+                                        const typename Storage<DT>::CT* bc_prof, const typename Storage<DT>::CT* bc_buf, int i,
                                         int step, int flags)
 {
     using CT = typename Storage<DT>::CT;
     pdl_wait(); // the gathered values
-    if (k >= n_nodes) return;
-    const int2 nd = nodes[k];
+    if (i >= n_nodes) return;
+    const int4 nd = nodes[i];
     const CaseArgs<CT>& a = cases[nd.y];
-    const int c = nd.x;
+    const int c = nd.x, k = nd.z;
     const int lab = a.label[c] & L_MASK;
     const int x = c % a.nx, y = (c / a.nx) % a.ny, z = c / (a.nx * a.ny);
     CT rho, ux, uy, uz;
@@ -933,6 +1107,10 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
     using CT = typename Storage<DT>::CT;
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    // the chunk's record, which no step changes, comes in while the step before drains
+    Chunk ch{};
+    if constexpr (!(PAIR && pairs_chunks(DT, COL)))
+        if (w < g.n_chunks) ch = g.chunks[w];
     if (g.n_gather == 0) pdl_wait();
     const int step = g.cursor[ODD ? 1 : 0];
     if (blockIdx.x == 0 && threadIdx.x == 0) g.cursor[ODD ? 0 : 1] = step + 1;
@@ -952,14 +1130,12 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
                 const bool adj = adjacent_span<DT>(ca, cb);
                 if (adj) pair_load_adjacent<DT, ODD>(a, ca.c0, lane, f);
                 else pair_load<DT, ODD>(a, ca, cb, lane, f);
-                pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * w, g.chunk_nodes + 2 * w, f, step, flags, lane,
-                                          adj);
+                pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * w, g.chunk_nodes, f, step, flags, lane, adj);
             } else {
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes + 2 * w, step, flags, lane);
+                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes, step, flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
-                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * w + 1,
-                                              g.chunk_nodes + 2 * w + 1, step, flags, lane);
+                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * w + 1, g.chunk_nodes, step, flags, lane);
                 }
             }
         } else {
@@ -967,9 +1143,8 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
         }
     } else {
         if (w < g.n_chunks) {
-            const Chunk ch = g.chunks[w];
             const int ci = ch.cflags & CH_CASE_MASK;
-            fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes + w, step, flags, lane);
+            fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, step, flags, lane);
         } else {
             node_batch<DT, ODD>(g.nodes, g.n_nodes, g.cases, g.bc_prof, g.bc_buf, (w - g.n_chunks) * 32 + lane, step, flags);
         }
@@ -1215,18 +1390,16 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
                 f2 f[27];
                 const bool adj = adjacent_span<DT>(ca, cb);
                 staged_pair_load<DT, ODD>(a, ca, cb, adj, lane, buffer(b), f);
-                pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * u, g.chunk_nodes + 2 * u, f, step, flags, lane,
-                                          adj);
+                pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * u, g.chunk_nodes, f, step, flags, lane, adj);
                 __syncwarp();
                 state = ls[1];
             } else {
                 // inline like the two-cell kernel's, so that both round these chunks alike
                 if (lane == 0) ls[1] = state;
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes + 2 * u, step, flags, lane);
+                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes, step, flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
-                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * u + 1,
-                                              g.chunk_nodes + 2 * u + 1, step, flags, lane);
+                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * u + 1, g.chunk_nodes, step, flags, lane);
                 }
                 __syncwarp();
                 state = ls[1];

@@ -441,12 +441,10 @@ __device__ __forceinline__ void cum_x_raw(const CumPost<CT>& s, CT irs, CT ux, C
     k[0][1][2] = CT(0); k[1][1][2] = s112; k[2][1][2] = ux * (s112 + s112);
 }
 
-template <class CT, int DT, bool PLANES, class PT>
-__device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy,
-                                            CT* S, CT sc, CT isc)
+template <class CT, int DT, bool PLANES>
+__device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, const Central<CT>& C, CT fx, CT fy, CT fz, CT nu, CT sc,
+                                            CT isc)
 {
-    const Central<CT> C = central_moments<CT>(c, fx, fy, fz);
-    if (cy) nu = cy_nu_from_central(C.xx, C.yy, C.zz, C.xy, C.xz, C.yz, c.rho, *cy, S);
     const CT om = CT(1) / (CT(3) * nu + CT(0.5));
     // relaxation (lbm_col_cum.h:205-235 with omega2 = 1): the shear parts by omega1, the trace
     // to rho; all times the storage scale
@@ -846,31 +844,34 @@ __device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx
 }
 
 // density, velocity (u = (j + F/2) / rho) and the collision of one cell's stored values g (or
-// of two cells', CT = f2).  With `cy` the shear viscosity is the local Carreau-Yasuda one and S
-// receives the strain rate.  PT: the type of the viscosity-law parameters
-template <class CT, int COL, int DT, bool PLANES, class PT>
-__device__ __forceinline__ void step_cell(CT* g, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, CT sc, CT isc, CT* S,
-                                          CT& rho, CT& ux, CT& uy, CT& uz)
+// of two cells', CT = f2).  With `cy` the shear viscosity is the local Carreau-Yasuda one.  PT: the
+// type of the viscosity-law parameters.  out(rho, ux, uy, uz, S) is called once they are known
+// (S: the strain rate with `cy`, else null), before the populations are rebuilt, so that
+// nothing of it is held in registers meanwhile
+template <class CT, int COL, int DT, bool PLANES, class PT, class Out>
+__device__ __forceinline__ void step_cell(CT* g, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, CT sc, CT isc, Out&& out)
 {
     constexpr bool KBC = COL >= COL_KBC_N1 && COL <= COL_KBC_C4;
     const CellState<CT> c = cell_state<CT, DT, PLANES, KBC>(g, fx, fy, fz, isc);
-    rho = c.rho; ux = c.ux; uy = c.uy; uz = c.uz;
-    if constexpr (COL == COL_CUM) {
-        collide_cum<CT, DT, PLANES, PT>(g, c, fx, fy, fz, nu, cy, S, sc, isc);
+    Central<CT> C;
+    if (COL == COL_CUM || cy) C = central_moments<CT>(c, fx, fy, fz);
+    if (cy) {
+        CT S[6];
+        nu = cy_nu_from_central(C.xx, C.yy, C.zz, C.xy, C.xz, C.yz, c.rho, *cy, S);
+        out(c.rho, c.ux, c.uy, c.uz, (const CT*)S);
     } else {
-        if (cy) {
-            const Central<CT> C = central_moments<CT>(c, fx, fy, fz);
-            nu = cy_nu_from_central(C.xx, C.yy, C.zz, C.xy, C.xz, C.yz, c.rho, *cy, S);
-        }
-        if constexpr (COL == COL_MRT) {
-            collide_mrt<CT, DT>(g, c, nu, sc);
-        } else if constexpr (COL == COL_BGK) {
-            collide_bgk<CT, DT, PLANES>(g, c, fx, fy, fz, nu, sc);
-        } else {
-            constexpr bool central = COL >= COL_KBC_C1;
-            constexpr int v = central ? COL - COL_KBC_C1 + 1 : COL - COL_KBC_N1 + 1;
-            collide_kbc<CT, DT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(g, c, fx, fy, fz, nu, sc);
-        }
+        out(c.rho, c.ux, c.uy, c.uz, (const CT*)nullptr);
+    }
+    if constexpr (COL == COL_CUM) {
+        collide_cum<CT, DT, PLANES>(g, c, C, fx, fy, fz, nu, sc, isc);
+    } else if constexpr (COL == COL_MRT) {
+        collide_mrt<CT, DT>(g, c, nu, sc);
+    } else if constexpr (COL == COL_BGK) {
+        collide_bgk<CT, DT, PLANES>(g, c, fx, fy, fz, nu, sc);
+    } else {
+        constexpr bool central = COL >= COL_KBC_C1;
+        constexpr int v = central ? COL - COL_KBC_C1 + 1 : COL - COL_KBC_N1 + 1;
+        collide_kbc<CT, DT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(g, c, fx, fy, fz, nu, sc);
     }
 }
 
