@@ -236,8 +236,9 @@ int nnlbm_get_stats(nnlbm_ctx* ctx, int ic, double* out, int64_t* n_accumulated)
  * by nnlbm_tcpc_labels), read by the near-wall test of wss_proxy_pa; NULL = no walls.
  * out: [20][nz][ny][nx] floats in file order: velocity (3), mean_velocity (3), lbm_rho,
  * pressure_pa, gamma_dot, nu_phys_m2_s, mu_phys_pa_s, wss_proxy_pa, turbulence_intensity,
- * rms_velocity, strain_diag_1_s (3), strain_shear_1_s (3).  Allocates a device buffer of
- * 20 floats per cell for the call. */
+ * rms_velocity, strain_diag_1_s (3), strain_shear_1_s (3).  Uses a device buffer of 20
+ * floats and a byte per cell, kept by the context for the next call up to 256 MiB and
+ * allocated for the call above that. */
 int nnlbm_output_fields(nnlbm_ctx* ctx, int ic, const double* params, const uint8_t* wall_flags, float* out);
 
 /* Canonical populations (see the layout note above).  Replaces: LBM::copyDFsToHost

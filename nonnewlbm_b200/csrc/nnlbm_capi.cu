@@ -6,12 +6,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/nnlbm.h"
@@ -228,6 +230,13 @@ struct nnlbm_ctx {
     // a status range that the next k_step_prologue clears (left by nnlbm_step for its first launch)
     unsigned long long* zero_next = nullptr;
     int zero_next_words = 0;
+    // results on their way to the caller's arrays (read_array): pinned buffers of kReadChunk
+    // bytes, the event after each one's copy, as many as the largest read so far could use
+    std::vector<char*> read_buf;
+    std::vector<cudaEvent_t> read_done;
+    // the device buffers of nnlbm_output_fields (wall flags, fields), kept up to kKeepOutputBytes
+    char* d_output = nullptr;
+    size_t output_bytes = 0;
     // the staged step's bounded waits (GroupArgs::stage_wait_ns, stage_pad)
     long long stage_wait_ns = 2000000000LL;
     int stage_pad = 0;
@@ -717,6 +726,124 @@ int run_group_steps(nnlbm_ctx* ctx, Group& g, int64_t n, int flags, bool use_gra
         }
     }
     finish_steps(ctx, g, n, flags);
+    return NNLBM_OK;
+}
+
+// ---------------------------------------------------------------------------------------
+// device arrays into the caller's (pageable) arrays, converted on the way.  One copy into a
+// temporary vector and one loop over it took 95 ms for a field of 26.5 M floats (106 MB at
+// 50 GB/s are 2 ms): a pageable copy goes through the driver's own staging, and every page of the
+// vector and of the caller's array is touched for the first time by one thread.  Here the array
+// passes through pinned buffers of kReadChunk bytes, copied ahead on the context's stream, and
+// up to kReadThreads threads convert a buffer each, once its copy has run.
+// ---------------------------------------------------------------------------------------
+constexpr size_t kReadChunk = size_t(1) << 20;
+constexpr int kReadThreads = 8;
+constexpr size_t kKeepOutputBytes = size_t(256) << 20;
+
+template <class S, class D>
+void convert_array(const S* in, D* out, size_t n)
+{
+    if constexpr (std::is_same<S, D>::value) memcpy(out, in, n * sizeof(S));
+    else
+        for (size_t i = 0; i < n; ++i) out[i] = (D)in[i];
+}
+
+int ensure_read_buffers(nnlbm_ctx* ctx, size_t n)
+{
+    while (ctx->read_buf.size() < n) {
+        char* b = nullptr;
+        cudaEvent_t e = nullptr;
+        CK(cudaMallocHost((void**)&b, kReadChunk));
+        const cudaError_t rc = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+        if (rc != cudaSuccess) {
+            cudaFreeHost(b);
+            return set_err(ctx, NNLBM_ERR_CUDA, "event creation failed: %s", cudaGetErrorString(rc));
+        }
+        ctx->read_buf.push_back(b);
+        ctx->read_done.push_back(e);
+    }
+    return NNLBM_OK;
+}
+
+// n elements of the device array `src` into `out`, behind everything on the context's stream;
+// returns once they are there
+template <class S, class D>
+int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
+{
+    constexpr size_t per = kReadChunk / sizeof(S);
+    const size_t chunks = (n + per - 1) / per;
+    if (chunks == 0) return NNLBM_OK;
+    const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::min<size_t>({(size_t)kReadThreads, (size_t)hw, chunks});
+    const size_t slots = std::min(2 * threads, chunks);
+    int rc = ensure_read_buffers(ctx, slots);
+    if (rc != NNLBM_OK) return rc;
+    auto count = [&](size_t k) { return std::min(per, n - k * per); };
+    std::atomic<size_t> issued{0}, next{0};
+    std::atomic<int> failed{(int)cudaSuccess};
+    std::vector<std::atomic<size_t>> free_from(slots); // slot k % slots is free once it holds k + 1
+    for (auto& f : free_from) f.store(0);
+    auto work = [&](bool other) {
+        if (other) {
+            const cudaError_t e = cudaSetDevice(ctx->device);
+            if (e != cudaSuccess) {
+                failed.store((int)e);
+                return;
+            }
+        }
+        for (;;) {
+            const size_t k = next.fetch_add(1);
+            if (k >= chunks) return;
+            while (issued.load(std::memory_order_acquire) <= k) {
+                if (failed.load() != cudaSuccess) return;
+                std::this_thread::yield();
+            }
+            const cudaError_t e = cudaEventSynchronize(ctx->read_done[k % slots]);
+            if (e != cudaSuccess) {
+                failed.store((int)e);
+                return;
+            }
+            convert_array(reinterpret_cast<const S*>(ctx->read_buf[k % slots]), out + k * per, count(k));
+            free_from[k % slots].store(k + 1, std::memory_order_release);
+        }
+    };
+    std::vector<std::thread> team;
+    try {
+        for (size_t t = 1; t < threads; ++t) team.emplace_back(work, true);
+    } catch (...) {
+        // fewer threads, or none: the calling thread converts what they do not
+    }
+    // the copies, each once its slot is free again.  With no team this thread converts in
+    // between, so that a slot it waits for is always one it has itself emptied
+    for (size_t k = 0; k < chunks && failed.load() == cudaSuccess; ++k) {
+        if (k >= slots) {
+            if (team.empty()) {
+                const size_t d = next.fetch_add(1);
+                const cudaError_t e = cudaEventSynchronize(ctx->read_done[d % slots]);
+                if (e != cudaSuccess) {
+                    failed.store((int)e);
+                    break;
+                }
+                convert_array(reinterpret_cast<const S*>(ctx->read_buf[d % slots]), out + d * per, count(d));
+                free_from[d % slots].store(d + 1);
+            }
+            while (free_from[k % slots].load(std::memory_order_acquire) != k - slots + 1 && failed.load() == cudaSuccess)
+                std::this_thread::yield();
+            if (failed.load() != cudaSuccess) break;
+        }
+        cudaError_t e = cudaMemcpyAsync(ctx->read_buf[k % slots], src + k * per, count(k) * sizeof(S), cudaMemcpyDeviceToHost,
+                                        ctx->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->read_done[k % slots], ctx->stream);
+        if (e != cudaSuccess) failed.store((int)e);
+        else issued.store(k + 1, std::memory_order_release);
+    }
+    work(false);
+    for (std::thread& t : team) t.join();
+    if (failed.load() != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream); // no copy still writes the buffers
+        return set_err(ctx, NNLBM_ERR_CUDA, "reading results back failed: %s", cudaGetErrorString((cudaError_t)failed.load()));
+    }
     return NNLBM_OK;
 }
 
@@ -1447,16 +1574,8 @@ int nnlbm_get_macro(nnlbm_ctx* ctx, int ic, int field, double* out)
         if ((rc = ensure_macro(ctx, c)) != NNLBM_OK) return rc;
         CK(cudaStreamSynchronize(ctx->stream));
     }
-    // the copies below run on the legacy stream: let the context's queued steps finish first
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (c.ct_bytes == 8) {
-        CK(cudaMemcpy(out, (char*)c.d_macro + (size_t)field * c.N * 8, (size_t)c.N * 8, cudaMemcpyDeviceToHost));
-    } else {
-        std::vector<float> tmp((size_t)c.N);
-        CK(cudaMemcpy(tmp.data(), (char*)c.d_macro + (size_t)field * c.N * 4, (size_t)c.N * 4, cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < tmp.size(); ++i) out[i] = tmp[i];
-    }
-    return NNLBM_OK;
+    if (c.ct_bytes == 8) return read_array(ctx, (const double*)c.d_macro + (size_t)field * c.N, out, (size_t)c.N);
+    return read_array(ctx, (const float*)c.d_macro + (size_t)field * c.N, out, (size_t)c.N);
 }
 
 int nnlbm_get_stats(nnlbm_ctx* ctx, int ic, double* out, int64_t* n_accumulated)
@@ -1469,15 +1588,7 @@ int nnlbm_get_stats(nnlbm_ctx* ctx, int ic, double* out, int64_t* n_accumulated)
     CK(cudaSetDevice(ctx->device));
     const size_t n = (size_t)6 * c.N;
     if (!c.d_stats) { memset(out, 0, n * sizeof(double)); return NNLBM_OK; }
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (c.d.stats_f64) {
-        CK(cudaMemcpy(out, c.d_stats, n * 8, cudaMemcpyDeviceToHost));
-    } else {
-        std::vector<float> tmp(n);
-        CK(cudaMemcpy(tmp.data(), c.d_stats, n * 4, cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < n; ++i) out[i] = tmp[i];
-    }
-    return NNLBM_OK;
+    return c.d.stats_f64 ? read_array(ctx, (const double*)c.d_stats, out, n) : read_array(ctx, (const float*)c.d_stats, out, n);
 }
 
 int nnlbm_import_stats(nnlbm_ctx* ctx, int ic, const double* in, int64_t n_accumulated)
@@ -1611,15 +1722,21 @@ int nnlbm_output_fields(nnlbm_ctx* ctx, int ic, const double* params, const uint
     CK(cudaSetDevice(ctx->device));
     if ((rc = ensure_macro(ctx, c)) != NNLBM_OK) return rc;
     const size_t N = (size_t)c.N;
-    uint8_t* d_wall = nullptr;
-    float* d_out = nullptr;
-    CK(cudaMalloc(&d_wall, N));
-    const cudaError_t e = cudaMalloc(&d_out, (size_t)kOutputValues * N * sizeof(float));
-    if (e != cudaSuccess) {
-        cudaFree(d_wall);
-        return set_err(ctx, NNLBM_ERR_OOM, "output buffer of %zu bytes: %s", (size_t)kOutputValues * N * sizeof(float),
-                       cudaGetErrorString(e));
+    // fields and wall flags in one buffer, kept for the next call where it is small
+    const size_t out_bytes = (size_t)kOutputValues * N * sizeof(float), need = out_bytes + N;
+    if (ctx->output_bytes < need) {
+        if (ctx->d_output) cudaFree(ctx->d_output);
+        ctx->d_output = nullptr;
+        ctx->output_bytes = 0;
+        const cudaError_t e = cudaMalloc((void**)&ctx->d_output, need);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return set_err(ctx, NNLBM_ERR_OOM, "output buffer of %zu bytes: %s", need, cudaGetErrorString(e));
+        }
+        ctx->output_bytes = need;
     }
+    float* const d_out = (float*)ctx->d_output;
+    uint8_t* const d_wall = (uint8_t*)ctx->d_output + out_bytes;
     // the field values of the last step that stored them, after every step still queued
     cudaError_t err = wall_flags ? cudaMemcpyAsync(d_wall, wall_flags, N, cudaMemcpyHostToDevice, ctx->stream)
                                  : cudaMemsetAsync(d_wall, 0, N, ctx->stream);
@@ -1627,13 +1744,15 @@ int nnlbm_output_fields(nnlbm_ctx* ctx, int ic, const double* params, const uint
         aux_launchers(c.d.dtype).output_fields(c.args.data(), p, d_wall, d_out, ctx->stream);
         err = cudaGetLastError();
     }
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(out, d_out, (size_t)kOutputValues * N * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    cudaFree(d_wall);
-    cudaFree(d_out);
-    if (err != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "output fields: %s", cudaGetErrorString(err));
-    return NNLBM_OK;
+    rc = err != cudaSuccess ? set_err(ctx, NNLBM_ERR_CUDA, "output fields: %s", cudaGetErrorString(err))
+                            : read_array(ctx, d_out, out, (size_t)kOutputValues * N);
+    if (ctx->output_bytes > kKeepOutputBytes) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(ctx->d_output);
+        ctx->d_output = nullptr;
+        ctx->output_bytes = 0;
+    }
+    return rc;
 }
 
 int nnlbm_autotune_flags(nnlbm_ctx* ctx, int flags)
@@ -1939,6 +2058,9 @@ int nnlbm_destroy(nnlbm_ctx* ctx)
         if (r.h) cudaFreeHost(r.h);
         if (r.done) cudaEventDestroy(r.done);
     }
+    for (char* b : ctx->read_buf) cudaFreeHost(b);
+    for (cudaEvent_t e : ctx->read_done) cudaEventDestroy(e);
+    if (ctx->d_output) cudaFree(ctx->d_output);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
