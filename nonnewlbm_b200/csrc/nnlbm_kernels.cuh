@@ -661,21 +661,39 @@ struct StepRegs {
 // the neighbour indices wrapped around the box, and with the bits of hwm for directions whose
 // neighbour is a wall.  For 16-bit storage out of line on a copy, so that the plain path has its
 // registers to itself (a box of FP16 cells between walls, 26.5 M: 780 us against 805 inline);
-// in line with FP32 and FP64 (FP32, 7.9 M cells: 289 us against 308 out of line; halfway
-// junction x0.6, MRT_LES: 15.8 against 16.5)
+// in line with FP32 and FP64 (FP32, 7.9 M cells: 289 us against 308 out of line).
+//
+// Addresses come from the plain path's slot bases, the cell's index and the sum of three per-axis
+// wrap offsets (zero for most cells), a reflected direction's from the cell's own slot.  With the
+// wall mask read before the wait for the step before, a halfway junction x0.6 (MRT_LES, every
+// chunk next to a wall) takes 20.3 us a step; with three wrapped coordinates and a 64-bit product
+// for each access, behind the mask's load, it took 24.6
+struct WrapOffsets {
+    int x[2], y[2], z[2]; // of the neighbours at +1 and -1
+    __device__ __forceinline__ WrapOffsets(int c, int yz, int nx, int ny, int nz)
+    {
+        const int cy = yz & 0xffff, cz = yz >> 16, cx = c - nx * (cy + cz * ny), sz = nx * ny, n = sz * nz;
+        x[0] = cx == nx - 1 ? -nx : 0; x[1] = cx == 0 ? nx : 0;
+        y[0] = cy == ny - 1 ? -sz : 0; y[1] = cy == 0 ? sz : 0;
+        z[0] = cz == nz - 1 ? -n : 0; z[1] = cz == 0 ? n : 0;
+    }
+    // of the neighbour at +c_q
+    __device__ __forceinline__ int at(int q) const
+    {
+        return (cxq(q) ? x[cxq(q) < 0] : 0) + ((cyq(q) ? y[cyq(q) < 0] : 0) + (czq(q) ? z[czq(q) < 0] : 0));
+    }
+};
 template <int DT>
 __device__ __forceinline__ void general_load(const CaseArgs<typename Storage<DT>::CT>& a, int c, int yz, uint32_t hwm,
                                              typename Storage<DT>::CT* f)
 {
     using S = Storage<DT>;
     using T = typename S::T;
-    const int y = yz & 0xffff, z = yz >> 16, x = c - a.nx * (y + z * a.ny);
-    const int64_t sy = a.nx, sz = (int64_t)a.nx * a.ny;
-    const T* p = (const T*)a.df;
+    const WrapOffsets w(c, yz, a.nx, a.ny, a.nz);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
-        const int64_t n = wrapc(x - cxq(q), a.nx) + sy * wrapc(y - cyq(q), a.ny) + sz * wrapc(z - czq(q), a.nz);
-        f[q] = S::raw(((hwm >> oppq(q)) & 1u) ? p[q * a.qstride + c] : p[oppq(q) * a.qstride + n]);
+        const bool wall = (hwm >> oppq(q)) & 1u;
+        f[q] = S::raw(((const T*)(wall ? a.slot_even[q] : odd_ld(a, q)))[c + (wall ? 0 : w.at(oppq(q)))]);
     }
 }
 template <int DT>
@@ -684,13 +702,11 @@ __device__ __forceinline__ void general_store(const CaseArgs<typename Storage<DT
 {
     using S = Storage<DT>;
     using T = typename S::T;
-    const int y = yz & 0xffff, z = yz >> 16, x = c - a.nx * (y + z * a.ny);
-    const int64_t sy = a.nx, sz = (int64_t)a.nx * a.ny;
-    T* p = (T*)a.df;
+    const WrapOffsets w(c, yz, a.nx, a.ny, a.nz);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
-        const int64_t n = wrapc(x + cxq(q), a.nx) + sy * wrapc(y + cyq(q), a.ny) + sz * wrapc(z + czq(q), a.nz);
-        p[((hwm >> q) & 1u) ? oppq(q) * a.qstride + c : q * a.qstride + n] = S::put(f[q]);
+        const bool wall = (hwm >> q) & 1u;
+        ((T*)(wall ? a.slot_even[oppq(q)] : a.slot_odd_st[q]))[c + (wall ? 0 : w.at(q))] = S::put(f[q]);
     }
 }
 template <int DT>
@@ -706,9 +722,17 @@ __device__ __noinline__ void general_store_call(const CaseArgs<typename Storage<
     general_store<DT>(*ap, c, yz, hwm, f);
 }
 
+// the wall mask of a lane's cell in the odd step, which no step changes: it can be read before
+// the step before has ended
+template <bool ODD, class CT>
+__device__ __forceinline__ uint32_t chunk_walls(const CaseArgs<CT>& a, const Chunk& ch, int lane)
+{
+    return ODD && (ch.cflags & CH_HW) && ((ch.fluid >> lane) & 1u) ? a.hw[ch.c0 + lane] : 0u;
+}
+
 template <int DT, int COL, bool ODD>
 __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>::CT>& a, const CaseArgs<typename Storage<DT>::CT>* ap,
-                                            const Chunk& ch, const Chunk* chp, const ChunkNodes* nodes, int step, int flags,
+                                            const Chunk& ch, const Chunk* chp, const ChunkNodes* nodes, uint32_t hwm, int step, int flags,
                                             int lane)
 {
     using S = Storage<DT>;
@@ -725,10 +749,10 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
     CT f[27]; // the stored values
     if (on) {
         if (general && DT < 2) {
-            general_load<DT>(a, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, f);
+            general_load<DT>(a, c, ch.yz, hwm, f);
         } else if (general) {
             CT t[27];
-            general_load_call<DT>(ap, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, t);
+            general_load_call<DT>(ap, c, ch.yz, hwm, t);
 #pragma unroll
             for (int q = 0; q < 27; ++q) f[q] = t[q];
         } else {
@@ -777,12 +801,12 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
         // the gather of this step reads the slots written below
         if (ch.cflags & CH_WAIT) pdl_wait();
         if (general && DT < 2) {
-            general_store<DT>(a, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, f);
+            general_store<DT>(a, c, ch.yz, hwm, f);
         } else if (general) {
             CT t[27];
 #pragma unroll
             for (int q = 0; q < 27; ++q) t[q] = f[q];
-            general_store_call<DT>(ap, c, ch.yz, (ch.cflags & CH_HW) ? a.hw[c] : 0u, t);
+            general_store_call<DT>(ap, c, ch.yz, hwm, t);
         } else {
             // slot opp(q) at c, or slot q at c + c_q
 #pragma unroll
@@ -1107,16 +1131,24 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
     using CT = typename Storage<DT>::CT;
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    // the chunk's record, which no step changes, comes in while the step before drains
+    // the chunk's record and wall masks, which no step changes, come in while the step before drains
+    constexpr bool pair = PAIR && pairs_chunks(DT, COL);
     Chunk ch{};
-    if constexpr (!(PAIR && pairs_chunks(DT, COL)))
-        if (w < g.n_chunks) ch = g.chunks[w];
+    uint32_t hwm = 0u;
+    if constexpr (!pair) {
+        if (w < g.n_chunks) {
+            ch = g.chunks[w];
+            hwm = chunk_walls<ODD>(case_args<ARGS>(g, ch.cflags & CH_CASE_MASK), ch, lane);
+        }
+    }
     if (g.n_gather == 0) pdl_wait();
     const int step = g.cursor[ODD ? 1 : 0];
     if (blockIdx.x == 0 && threadIdx.x == 0) g.cursor[ODD ? 0 : 1] = step + 1;
-    // the step's flags are the same for every case of the group
+    // the step's flags are the same for every case of the group.  They are read ahead of the
+    // populations: after them (and the cursor stored last), a box of 192x144x120 FP32 cells took
+    // 167 us a step against 156, a junction 30.3 against 28.4
     const int flags = case_args<ARGS>(g, 0).ctl[step].flags;
-    if constexpr (PAIR && pairs_chunks(DT, COL)) {
+    if constexpr (pair) {
         // warp w takes chunks 2w and 2w + 1 (the host pads the list to an even length); a
         // pair that is not pairable (a face chunk, two cases, the finite-difference force)
         // is stepped chunk by chunk
@@ -1132,10 +1164,13 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
                 else pair_load<DT, ODD>(a, ca, cb, lane, f);
                 pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * w, g.chunk_nodes, f, step, flags, lane, adj);
             } else {
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes, step, flags, lane);
+                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
+                                          flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
-                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * w + 1, g.chunk_nodes, step, flags, lane);
+                    const CaseArgs<CT>& b = case_args<ARGS>(g, cj);
+                    fluid_chunk<DT, COL, ODD>(b, g.cases + cj, cb, g.chunks + 2 * w + 1, g.chunk_nodes, chunk_walls<ODD>(b, cb, lane),
+                                              step, flags, lane);
                 }
             }
         } else {
@@ -1144,7 +1179,7 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
     } else {
         if (w < g.n_chunks) {
             const int ci = ch.cflags & CH_CASE_MASK;
-            fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, step, flags, lane);
+            fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, hwm, step, flags, lane);
         } else {
             node_batch<DT, ODD>(g.nodes, g.n_nodes, g.cases, g.bc_prof, g.bc_buf, (w - g.n_chunks) * 32 + lane, step, flags);
         }
@@ -1396,10 +1431,13 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
             } else {
                 // inline like the two-cell kernel's, so that both round these chunks alike
                 if (lane == 0) ls[1] = state;
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes, step, flags, lane);
+                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
+                                          flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
-                    fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, cj), g.cases + cj, cb, g.chunks + 2 * u + 1, g.chunk_nodes, step, flags, lane);
+                    const CaseArgs<float>& e = case_args<ARGS>(g, cj);
+                    fluid_chunk<DT, COL, ODD>(e, g.cases + cj, cb, g.chunks + 2 * u + 1, g.chunk_nodes, chunk_walls<ODD>(e, cb, lane),
+                                              step, flags, lane);
                 }
                 __syncwarp();
                 state = ls[1];
