@@ -53,8 +53,9 @@ __global__ void k_init_macro(const CaseArgs<typename Storage<DT>::CT> a, typenam
     }
 }
 
-template <bool ODD, int ARGS>
-static void launch_gather(bool chained, dim3 grid, dim3 block, cudaStream_t s, const GroupArgs<typename Storage<NNLBM_DT>::CT>& g)
+// `kernel` for the group's argument mode; `chained`: a programmatic dependent of the kernel before
+template <class CT>
+static void launch_chained(void (*kernel)(GroupArgs<CT>), bool chained, dim3 grid, dim3 block, cudaStream_t s, const GroupArgs<CT>& g)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -65,39 +66,42 @@ static void launch_gather(bool chained, dim3 grid, dim3 block, cudaStream_t s, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = chained ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, &k_bc_gather<NNLBM_DT, ODD, ARGS>, g);
+    cudaLaunchKernelEx(&cfg, kernel, g);
 }
+
 void NNLBM_CAT(launch_bc_gather_, NNLBM_DT)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* args)
 {
     using CT = typename Storage<NNLBM_DT>::CT;
+    constexpr int DT = NNLBM_DT;
     const GroupArgs<CT>& g = *(const GroupArgs<CT>*)args;
-    switch (args_mode(g.n_cases)) {
-    case ARGS_ONE:
-        if (odd) launch_gather<true, ARGS_ONE>(chained, grid, block, s, g);
-        else launch_gather<false, ARGS_ONE>(chained, grid, block, s, g);
-        break;
-    case ARGS_PARAM:
-        if (odd) launch_gather<true, ARGS_PARAM>(chained, grid, block, s, g);
-        else launch_gather<false, ARGS_PARAM>(chained, grid, block, s, g);
-        break;
-    default:
-        if (odd) launch_gather<true, ARGS_GLOBAL>(chained, grid, block, s, g);
-        else launch_gather<false, ARGS_GLOBAL>(chained, grid, block, s, g);
-    }
+    const int mode = args_mode(g.n_cases);
+    launch_chained<CT>(mode == ARGS_ONE     ? (odd ? k_bc_gather<DT, true, ARGS_ONE> : k_bc_gather<DT, false, ARGS_ONE>)
+                       : mode == ARGS_PARAM ? (odd ? k_bc_gather<DT, true, ARGS_PARAM> : k_bc_gather<DT, false, ARGS_PARAM>)
+                                            : (odd ? k_bc_gather<DT, true, ARGS_GLOBAL> : k_bc_gather<DT, false, ARGS_GLOBAL>),
+                       chained, grid, block, s, g);
 }
 
-void NNLBM_CAT(launch_refd_velocity_, NNLBM_DT)(bool odd, dim3 grid, dim3 block, cudaStream_t s, const void* args)
+void NNLBM_CAT(launch_refd_velocity_, NNLBM_DT)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* args)
+{
+    using CT = typename Storage<NNLBM_DT>::CT;
+    constexpr int DT = NNLBM_DT;
+    const GroupArgs<CT>& g = *(const GroupArgs<CT>*)args;
+    const int mode = args_mode(g.n_cases);
+    launch_chained<CT>(mode == ARGS_ONE     ? (odd ? k_refd_velocity<DT, true, ARGS_ONE> : k_refd_velocity<DT, false, ARGS_ONE>)
+                       : mode == ARGS_PARAM ? (odd ? k_refd_velocity<DT, true, ARGS_PARAM> : k_refd_velocity<DT, false, ARGS_PARAM>)
+                                            : (odd ? k_refd_velocity<DT, true, ARGS_GLOBAL> : k_refd_velocity<DT, false, ARGS_GLOBAL>),
+                       chained, grid, block, s, g);
+}
+
+void NNLBM_CAT(launch_refd_stress_, NNLBM_DT)(bool, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* args)
 {
     using CT = typename Storage<NNLBM_DT>::CT;
     const GroupArgs<CT>& g = *(const GroupArgs<CT>*)args;
-    if (odd) k_refd_velocity<NNLBM_DT, true><<<grid, block, 0, s>>>(g);
-    else k_refd_velocity<NNLBM_DT, false><<<grid, block, 0, s>>>(g);
-}
-
-void NNLBM_CAT(launch_refd_stress_, NNLBM_DT)(bool, dim3 grid, dim3 block, cudaStream_t s, const void* args)
-{
-    using CT = typename Storage<NNLBM_DT>::CT;
-    k_refd_stress<CT><<<grid, block, 0, s>>>(*(const GroupArgs<CT>*)args);
+    const int mode = args_mode(g.n_cases);
+    launch_chained<CT>(mode == ARGS_ONE     ? k_refd_stress<CT, ARGS_ONE>
+                       : mode == ARGS_PARAM ? k_refd_stress<CT, ARGS_PARAM>
+                                            : k_refd_stress<CT, ARGS_GLOBAL>,
+                       chained, grid, block, s, g);
 }
 
 void NNLBM_CAT(launch_fill_eq_, NNLBM_DT)(const void* args, double rho, double ux, double uy, double uz, cudaStream_t s)
@@ -126,8 +130,11 @@ cudaError_t NNLBM_CAT(load_bc_, NNLBM_DT)()
     const void* fns[] = {(const void*)k_bc_gather<NNLBM_DT, false, ARGS_ONE>, (const void*)k_bc_gather<NNLBM_DT, true, ARGS_ONE>,
                          (const void*)k_bc_gather<NNLBM_DT, false, ARGS_PARAM>, (const void*)k_bc_gather<NNLBM_DT, true, ARGS_PARAM>,
                          (const void*)k_bc_gather<NNLBM_DT, false, ARGS_GLOBAL>, (const void*)k_bc_gather<NNLBM_DT, true, ARGS_GLOBAL>,
-                         (const void*)k_refd_velocity<NNLBM_DT, false>, (const void*)k_refd_velocity<NNLBM_DT, true>,
-                         (const void*)k_refd_stress<CT>, (const void*)k_fill_eq<NNLBM_DT>, (const void*)k_init_macro<NNLBM_DT>,
+                         (const void*)k_refd_velocity<NNLBM_DT, false, ARGS_ONE>, (const void*)k_refd_velocity<NNLBM_DT, true, ARGS_ONE>,
+                         (const void*)k_refd_velocity<NNLBM_DT, false, ARGS_PARAM>, (const void*)k_refd_velocity<NNLBM_DT, true, ARGS_PARAM>,
+                         (const void*)k_refd_velocity<NNLBM_DT, false, ARGS_GLOBAL>, (const void*)k_refd_velocity<NNLBM_DT, true, ARGS_GLOBAL>,
+                         (const void*)k_refd_stress<CT, ARGS_ONE>, (const void*)k_refd_stress<CT, ARGS_PARAM>,
+                         (const void*)k_refd_stress<CT, ARGS_GLOBAL>, (const void*)k_fill_eq<NNLBM_DT>, (const void*)k_init_macro<NNLBM_DT>,
                          (const void*)k_output_fields<CT>};
     cudaFuncAttributes fa;
     for (const void* f : fns) {

@@ -31,8 +31,8 @@ namespace nnlbm {
 NNLBM_DECL_STEP_DT(0) NNLBM_DECL_STEP_DT(1) NNLBM_DECL_STEP_DT(2) NNLBM_DECL_STEP_DT(3)
 #define NNLBM_DECL_AUX(DT)                                                                \
     void launch_bc_gather_##DT(bool, bool, dim3, dim3, cudaStream_t, const void*);       \
-    void launch_refd_velocity_##DT(bool, dim3, dim3, cudaStream_t, const void*);         \
-    void launch_refd_stress_##DT(bool, dim3, dim3, cudaStream_t, const void*);           \
+    void launch_refd_velocity_##DT(bool, bool, dim3, dim3, cudaStream_t, const void*);   \
+    void launch_refd_stress_##DT(bool, bool, dim3, dim3, cudaStream_t, const void*);     \
     void launch_fill_eq_##DT(const void*, double, double, double, double, cudaStream_t); \
     void launch_init_macro_##DT(const void*, double, double, double, double, cudaStream_t); \
     void launch_output_fields_##DT(const void*, const OutputParams&, const uint8_t*, float*, cudaStream_t); \
@@ -73,8 +73,7 @@ StagedOccupancy staged_occupancy(int dt, int col)
 }
 
 struct AuxLaunchers {
-    void (*gather)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* group_args);
-    GroupLauncher refd_velocity, refd_stress;
+    GroupLauncher gather, refd_velocity, refd_stress;
     void (*fill_eq)(const void*, double, double, double, double, cudaStream_t);
     void (*init_macro)(const void*, double, double, double, double, cudaStream_t);
     void (*output_fields)(const void*, const OutputParams&, const uint8_t*, float*, cudaStream_t);
@@ -556,8 +555,8 @@ int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool o
     auto blocks = [](int warps, int per) { return dim3(std::max((warps + per - 1) / per, 1)); };
     if (!only_step && g.any_refd) {
         const dim3 rgrid = blocks(g.n_chunks, per_block); // one warp per chunk
-        A.refd_velocity(odd, rgrid, dim3(g.block), ctx->stream, args);
-        A.refd_stress(odd, rgrid, dim3(g.block), ctx->stream, args);
+        A.refd_velocity(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
+        A.refd_stress(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
     }
     if (!only_step && g.n_gather > 0) A.gather(odd, chained, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     dim3 grid = blocks(step_warps(g), per_block), block(g.block);
@@ -1919,9 +1918,9 @@ int nnlbm_profile_step(nnlbm_ctx* ctx, int ic, int64_t n_steps, int flags, doubl
         const bool odd = ((parity + k) & 1) != 0;
         if (mark(-1)) return set_err(ctx, NNLBM_ERR_CUDA, "event record failed");
         if (g.any_refd) {
-            A.refd_velocity(odd, rgrid, cblk, ctx->stream, g.args.data());
+            A.refd_velocity(odd, false, rgrid, cblk, ctx->stream, g.args.data());
             mark(3);
-            A.refd_stress(odd, rgrid, cblk, ctx->stream, g.args.data());
+            A.refd_stress(odd, false, rgrid, cblk, ctx->stream, g.args.data());
             mark(4);
         }
         if (g.n_gather > 0) {

@@ -223,7 +223,8 @@ __host__ __device__ constexpr int args_mode(int n_cases)
 
 // Programmatic dependent launch: the kernels of a step, and the steps of a call, are chained, so
 // that the launch of each overlaps the end of the one before.  A step launches the open-plane
-// gather, where it has nodes to gather, and the step kernel.
+// gather, where it has nodes to gather, and the step kernel; with the finite-difference
+// Carreau-Yasuda coupling its velocity and strain kernels first, each waiting for the one before.
 //   - The first kernel of a step waits for the step before as its first act.
 //   - The gather then lets the step kernel start at once.  The slots that it reads are
 //     overwritten by the step: the chunks that hold them (CH_WAIT) and the node warps wait for
@@ -1553,23 +1554,33 @@ __global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupA
 // of every FLUID cell with the force of the previous step, then the finite-difference
 // strain from it.  Non-FLUID values are never read by the strain stencil.
 // ---------------------------------------------------------------------------------------
-template <int DT, bool ODD>
+//
+// Both are chained to the kernels around them; what no step changes (chunk record, wall masks,
+// labels) is read before the wait.  A FLUID cell lies off every face, so its pull is the step's own:
+// slot q at the cell (even) or slot opp(q) at x - c_q (odd), a population that a wall reflects
+// from slot q at the cell in both; the slot bases of the step give all 27 addresses.  A step of a
+// junction x0.5 (FP32, four kernels): 31.3 -> 28.7 us against clamped and wrapped coordinates for
+// every population and launches that waited for one another's end.
+template <int DT, bool ODD, int ARGS>
 __global__ void __launch_bounds__(256) k_refd_velocity(const __grid_constant__ GroupArgs<typename Storage<DT>::CT> g)
 {
-    using CT = typename Storage<DT>::CT;
+    using S = Storage<DT>;
+    using CT = typename S::CT;
     const int lane = threadIdx.x & 31;
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (warp >= g.n_chunks) return;
-    const Chunk& ch = g.chunks[warp];
-    const CaseArgs<CT>& a = g.cases[ch.cflags & CH_CASE_MASK];
-    if (a.cy_mode != CY_REF_FD) return;
-    const int y = ch.yz & 0xffff, z = ch.yz >> 16;
-    const int x = ch.c0 - y * a.nx - z * a.nx * a.ny + lane;
+    Chunk ch{};
+    if (warp < g.n_chunks) ch = g.chunks[warp];
+    const CaseArgs<CT>& a = case_args<ARGS>(g, ch.cflags & CH_CASE_MASK);
+    const uint32_t hwm = chunk_walls<ODD>(a, ch, lane);
+    pdl_wait();
+    if (a.cy_mode != CY_REF_FD || !((ch.fluid & ~ch.periodic) >> lane & 1u)) return;
     const int c = ch.c0 + lane;
-    if (x >= a.nx || (a.label[c] & L_MASK) != L_FLUID) return;
-    const int xs[3] = {x - 1, x, x + 1}, ys[3] = {y - 1, y, y + 1}, zs[3] = {z - 1, z, z + 1};
     CT f[27];
-    pull_triples<DT, ODD>(a, xs, ys, zs, f);
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const bool own = !ODD || ((hwm >> oppq(q)) & 1u);
+        f[q] = S::load((const typename S::T*)(own ? a.slot_even[q] : odd_ld(a, q)), c, q, a.inv_scale);
+    }
     CT* M = a.macro;
     const int64_t N = a.N;
     CT rho, ux, uy, uz;
@@ -1577,26 +1588,26 @@ __global__ void __launch_bounds__(256) k_refd_velocity(const __grid_constant__ G
     M[M_RHO * N + c] = rho; M[M_VX * N + c] = ux; M[M_VY * N + c] = uy; M[M_VZ * N + c] = uz;
 }
 
-template <class CT>
+template <class CT, int ARGS>
 __global__ void __launch_bounds__(256) k_refd_stress(const __grid_constant__ GroupArgs<CT> g)
 {
     const int lane = threadIdx.x & 31;
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (warp >= g.n_chunks) return;
-    const Chunk& ch = g.chunks[warp];
-    const CaseArgs<CT>& a = g.cases[ch.cflags & CH_CASE_MASK];
-    if (a.cy_mode != CY_REF_FD) return;
-    const int sy = a.nx, sz = a.nx * a.ny;
-    const int y = ch.yz & 0xffff, z = ch.yz >> 16;
-    const int x = ch.c0 - y * sy - z * sz + lane;
-    const int c = ch.c0 + lane;
-    if (x >= a.nx || (a.label[c] & L_MASK) != L_FLUID) return;
-    CT* M = a.macro;
-    const int64_t N = a.N;
+    Chunk ch{};
+    if (warp < g.n_chunks) ch = g.chunks[warp];
+    const CaseArgs<CT>& a = case_args<ARGS>(g, ch.cflags & CH_CASE_MASK);
+    const int sy = a.nx, sz = a.nx * a.ny, c = ch.c0 + lane;
+    const bool on = a.cy_mode == CY_REF_FD && ((ch.fluid & ~ch.periodic) >> lane & 1u);
     const int cn[6] = {c - 1, c + 1, c - sy, c + sy, c - sz, c + sz};
     bool fl[6];
+    if (on) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) fl[k] = (a.label[cn[k]] & L_MASK) == L_FLUID;
+        for (int k = 0; k < 6; ++k) fl[k] = (a.label[cn[k]] & L_MASK) == L_FLUID;
+    }
+    pdl_wait();
+    if (!on) return;
+    CT* M = a.macro;
+    const int64_t N = a.N;
     auto d1 = [&](int fld, int axis) -> CT {
         const bool m = fl[2 * axis], p = fl[2 * axis + 1];
         const CT* F = M + (int64_t)fld * N;
@@ -1675,12 +1686,12 @@ __global__ void __launch_bounds__(256) k_output_fields(const CaseArgs<CT> a, con
 // host-side dispatch: one function per (storage, collision) instantiated in its own
 // translation unit
 // ---------------------------------------------------------------------------------------
-using GroupLauncher = void (*)(bool odd, dim3 grid, dim3 block, cudaStream_t s, const void* group_args);
+// (`chained`: launched as a programmatic dependent of the kernel just enqueued on the stream)
+using GroupLauncher = void (*)(bool odd, bool chained, dim3 grid, dim3 block, cudaStream_t s, const void* group_args);
 // the step kernel's launch forms: one cell a thread, two (the paired form), and the paired
 // form with staged loads (k_step_staged, persistent warps, StageGeom shared memory)
 enum : int { FORM_ONE = 0, FORM_PAIRED = 1, FORM_STAGED = 2 };
-// the step kernel's launcher: `chained` launches it as a programmatic dependent of the kernel
-// just enqueued on the stream
+// the step kernel's launcher
 using StepLauncher = void (*)(bool odd, bool chained, int form, dim3 grid, dim3 block, cudaStream_t s,
                               const void* group_args);
 // resident blocks per SM of the staged form (0 where the variant has no staged form)
