@@ -229,9 +229,9 @@ struct nnlbm_ctx {
     // a status range that the next k_step_prologue clears (left by nnlbm_step for its first launch)
     unsigned long long* zero_next = nullptr;
     int zero_next_words = 0;
-    // results on their way to the caller's arrays (read_array): pinned buffers of kReadChunk
-    // bytes, the event after each one's copy, as many as the largest read so far could use
-    std::vector<char*> read_buf;
+    // results on their way to the caller's arrays (read_array): kReadSlots pinned buffers of
+    // kReadChunk bytes, the event after each one's copy
+    char* read_buf = nullptr;
     std::vector<cudaEvent_t> read_done;
     // the device buffers of nnlbm_output_fields (wall flags, fields), kept up to kKeepOutputBytes
     char* d_output = nullptr;
@@ -733,11 +733,17 @@ int run_group_steps(nnlbm_ctx* ctx, Group& g, int64_t n, int flags, bool use_gra
 // temporary vector and one loop over it took 95 ms for a field of 26.5 M floats (106 MB at
 // 50 GB/s are 2 ms): a pageable copy goes through the driver's own staging, and every page of the
 // vector and of the caller's array is touched for the first time by one thread.  Here the array
-// passes through pinned buffers of kReadChunk bytes, copied ahead on the context's stream, and
-// up to kReadThreads threads convert a buffer each, once its copy has run.
+// passes through kReadSlots pinned buffers, one allocation that a context makes at its first large
+// read; the calling thread copies ahead and waits for the copies, and of an array of kReadAlone
+// buffers or more other threads, one for every kReadPerThread and at most kReadThreads, convert.
+// They make no CUDA call.  Below that the calling thread converts alone: with 5 to 7 threads on 16
+// cores that a program's own thread pool keeps busy too, 32 fields of 2 M floats took 119-136 ms
+// against 97 by one.  An array of up to kReadSmall bytes takes the pageable copy (its
+// pinned buffer cost a new context 11 ms)
 // ---------------------------------------------------------------------------------------
-constexpr size_t kReadChunk = size_t(1) << 20;
-constexpr int kReadThreads = 8;
+constexpr size_t kReadChunk = size_t(1) << 19;
+constexpr size_t kReadSlots = 8, kReadAlone = 32, kReadPerThread = 12, kReadThreads = 7;
+constexpr size_t kReadSmall = size_t(2) << 20;
 constexpr size_t kKeepOutputBytes = size_t(256) << 20;
 
 template <class S, class D>
@@ -748,20 +754,14 @@ void convert_array(const S* in, D* out, size_t n)
         for (size_t i = 0; i < n; ++i) out[i] = (D)in[i];
 }
 
-int ensure_read_buffers(nnlbm_ctx* ctx, size_t n)
+int ensure_read_buffers(nnlbm_ctx* ctx)
 {
-    while (ctx->read_buf.size() < n) {
-        char* b = nullptr;
+    while (ctx->read_done.size() < kReadSlots) {
         cudaEvent_t e = nullptr;
-        CK(cudaMallocHost((void**)&b, kReadChunk));
-        const cudaError_t rc = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-        if (rc != cudaSuccess) {
-            cudaFreeHost(b);
-            return set_err(ctx, NNLBM_ERR_CUDA, "event creation failed: %s", cudaGetErrorString(rc));
-        }
-        ctx->read_buf.push_back(b);
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         ctx->read_done.push_back(e);
     }
+    if (!ctx->read_buf) CK(cudaMallocHost((void**)&ctx->read_buf, kReadSlots * kReadChunk));
     return NNLBM_OK;
 }
 
@@ -770,78 +770,77 @@ int ensure_read_buffers(nnlbm_ctx* ctx, size_t n)
 template <class S, class D>
 int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
 {
+    if (n * sizeof(S) <= kReadSmall) {
+        std::vector<S> tmp;
+        S* to = nullptr;
+        if constexpr (std::is_same<S, D>::value) to = out;
+        else {
+            tmp.resize(n);
+            to = tmp.data();
+        }
+        CK(cudaMemcpyAsync(to, src, n * sizeof(S), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if constexpr (!std::is_same<S, D>::value) convert_array(to, out, n);
+        return NNLBM_OK;
+    }
+    const int rc = ensure_read_buffers(ctx);
+    if (rc != NNLBM_OK) return rc;
     constexpr size_t per = kReadChunk / sizeof(S);
     const size_t chunks = (n + per - 1) / per;
-    if (chunks == 0) return NNLBM_OK;
-    const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const size_t threads = std::min<size_t>({(size_t)kReadThreads, (size_t)hw, chunks});
-    const size_t slots = std::min(2 * threads, chunks);
-    int rc = ensure_read_buffers(ctx, slots);
-    if (rc != NNLBM_OK) return rc;
-    auto count = [&](size_t k) { return std::min(per, n - k * per); };
-    std::atomic<size_t> issued{0}, next{0};
-    std::atomic<int> failed{(int)cudaSuccess};
-    std::vector<std::atomic<size_t>> free_from(slots); // slot k % slots is free once it holds k + 1
-    for (auto& f : free_from) f.store(0);
-    auto work = [&](bool other) {
-        if (other) {
-            const cudaError_t e = cudaSetDevice(ctx->device);
-            if (e != cudaSuccess) {
-                failed.store((int)e);
-                return;
-            }
-        }
-        for (;;) {
-            const size_t k = next.fetch_add(1);
-            if (k >= chunks) return;
-            while (issued.load(std::memory_order_acquire) <= k) {
-                if (failed.load() != cudaSuccess) return;
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = chunks < kReadAlone ? 0 : std::min({kReadThreads, hw / 2, chunks / kReadPerThread});
+    std::atomic<size_t> ready{0}, next{0};
+    std::atomic<bool> failed{false};
+    std::atomic<size_t> converted[kReadSlots]; // slot k % kReadSlots: k + 1 once chunk k is out of it
+    for (auto& v : converted) v.store(0);
+    auto convert = [&](size_t k) {
+        const char* b = ctx->read_buf + (k % kReadSlots) * kReadChunk;
+        convert_array(reinterpret_cast<const S*>(b), out + k * per, std::min(per, n - k * per));
+        converted[k % kReadSlots].store(k + 1, std::memory_order_release);
+    };
+    auto work = [&] {
+        for (size_t k; (k = next.fetch_add(1)) < chunks;) {
+            while (ready.load(std::memory_order_acquire) <= k) {
+                if (failed.load()) return;
                 std::this_thread::yield();
             }
-            const cudaError_t e = cudaEventSynchronize(ctx->read_done[k % slots]);
-            if (e != cudaSuccess) {
-                failed.store((int)e);
-                return;
-            }
-            convert_array(reinterpret_cast<const S*>(ctx->read_buf[k % slots]), out + k * per, count(k));
-            free_from[k % slots].store(k + 1, std::memory_order_release);
+            convert(k);
         }
     };
     std::vector<std::thread> team;
     try {
-        for (size_t t = 1; t < threads; ++t) team.emplace_back(work, true);
+        team.reserve(threads);
+        for (size_t t = 0; t < threads; ++t) team.emplace_back(work);
     } catch (...) {
-        // fewer threads, or none: the calling thread converts what they do not
+        // fewer threads, or none: then this thread converts
     }
-    // the copies, each once its slot is free again.  With no team this thread converts in
-    // between, so that a slot it waits for is always one it has itself emptied
-    for (size_t k = 0; k < chunks && failed.load() == cudaSuccess; ++k) {
-        if (k >= slots) {
-            if (team.empty()) {
-                const size_t d = next.fetch_add(1);
-                const cudaError_t e = cudaEventSynchronize(ctx->read_done[d % slots]);
-                if (e != cudaSuccess) {
-                    failed.store((int)e);
-                    break;
-                }
-                convert_array(reinterpret_cast<const S*>(ctx->read_buf[d % slots]), out + d * per, count(d));
-                free_from[d % slots].store(d + 1);
-            }
-            while (free_from[k % slots].load(std::memory_order_acquire) != k - slots + 1 && failed.load() == cudaSuccess)
+    // chunk k is copied once its slot is empty, as far ahead as there are slots
+    cudaError_t e = cudaSuccess;
+    size_t issued = 0;
+    for (size_t k = 0; k < chunks && e == cudaSuccess; ++k) {
+        while (issued < chunks && issued < k + kReadSlots && e == cudaSuccess) {
+            const size_t slot = issued % kReadSlots;
+            if (issued >= kReadSlots && converted[slot].load(std::memory_order_acquire) != issued - kReadSlots + 1) {
+                if (issued > k) break; // chunk k is on its way: hand it over first
                 std::this_thread::yield();
-            if (failed.load() != cudaSuccess) break;
+                continue;
+            }
+            e = cudaMemcpyAsync(ctx->read_buf + slot * kReadChunk, src + issued * per, std::min(per, n - issued * per) * sizeof(S),
+                                cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->read_done[slot], ctx->stream);
+            if (e == cudaSuccess) ++issued;
         }
-        cudaError_t e = cudaMemcpyAsync(ctx->read_buf[k % slots], src + k * per, count(k) * sizeof(S), cudaMemcpyDeviceToHost,
-                                        ctx->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->read_done[k % slots], ctx->stream);
-        if (e != cudaSuccess) failed.store((int)e);
-        else issued.store(k + 1, std::memory_order_release);
+        if (e == cudaSuccess) e = cudaEventSynchronize(ctx->read_done[k % kReadSlots]);
+        if (e != cudaSuccess) break;
+        ready.store(k + 1, std::memory_order_release);
+        if (team.empty()) convert(k);
     }
-    work(false);
+    if (e != cudaSuccess) failed.store(true);
+    else if (!team.empty()) work();
     for (std::thread& t : team) t.join();
-    if (failed.load() != cudaSuccess) {
+    if (e != cudaSuccess) {
         cudaStreamSynchronize(ctx->stream); // no copy still writes the buffers
-        return set_err(ctx, NNLBM_ERR_CUDA, "reading results back failed: %s", cudaGetErrorString((cudaError_t)failed.load()));
+        return set_err(ctx, NNLBM_ERR_CUDA, "reading results back failed: %s", cudaGetErrorString(e));
     }
     return NNLBM_OK;
 }
@@ -2057,7 +2056,7 @@ int nnlbm_destroy(nnlbm_ctx* ctx)
         if (r.h) cudaFreeHost(r.h);
         if (r.done) cudaEventDestroy(r.done);
     }
-    for (char* b : ctx->read_buf) cudaFreeHost(b);
+    if (ctx->read_buf) cudaFreeHost(ctx->read_buf);
     for (cudaEvent_t e : ctx->read_done) cudaEventDestroy(e);
     if (ctx->d_output) cudaFree(ctx->d_output);
     if (ctx->d_status) cudaFree(ctx->d_status);
