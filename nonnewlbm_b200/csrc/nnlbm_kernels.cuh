@@ -617,28 +617,36 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
     return dt != 0 && (col == COL_CUM || col == COL_BGK || col == COL_MRT);
 }
 
-// register budget per thread of each step-kernel variant: FP64 arithmetic may use all
-// 255; the paired form (two cells per thread) gets NNLBM_PAIR_REGS (two 256-thread blocks
-// per SM); the one-cell form of a collision that can pair gets NNLBM_CHUNK_REGS_F32 with
-// FP32 storage (80, the most that keeps three blocks: the step then spills almost nothing,
-// which outweighs the lost warps) and
-// NNLBM_CHUNK_REGS with FP16/BF16 storage (four blocks: the packed loads need fewer
-// registers, and the extra warps hide the conversions); KBC, which never pairs, 128
+// register budget per thread of each step-kernel variant.  FP64 arithmetic may use all 255; the
+// paired form (two cells per thread) gets NNLBM_PAIR_REGS (two 256-thread blocks per SM).  The
+// one-cell forms run in 64-thread blocks, so that the budget sets the warps per SM almost
+// continuously, and a few spilled values cost less than the warps that hide the loads; us a step
+// by budget, one B200:
+//   FP32 storage, NNLBM_CHUNK_REGS_F32       72     80     88     96
+//     cumulant, box 192x144x120             151    167    172    174
+//     with mean/rms sums                    195    196    196    205
+//     BGK / MRT_LES, 211x163x137        214/211 226/228 238/230 232/232
+//   16-bit cumulant, NNLBM_CHUNK_REGS_CUM16  64     72     80     88
+//     box 384x288x240, FP16                 859    881    999   1080
+//   KBC, NNLBM_KBC_REGS                      80     96    104    128
+//     KBC_N4 / N1, FP32 box 176x144x112 183/173 211/200 209/199 208/199
+//     KBC_N4 FP16 junction x0.75           18.5   19.4   19.0   18.7
+// 16-bit BGK and MRT_LES keep NNLBM_CHUNK_REGS: autotuned, 180.9 to 181.9 us at 64 to 96 on the box
+// of 211x163x137
 #ifndef NNLBM_PAIR_REGS
 #define NNLBM_PAIR_REGS 128
 #endif
 #ifndef NNLBM_KBC_REGS
-#define NNLBM_KBC_REGS 128
+#define NNLBM_KBC_REGS 80
 #endif
 #ifndef NNLBM_CHUNK_REGS
 #define NNLBM_CHUNK_REGS 64
 #endif
 #ifndef NNLBM_CHUNK_REGS_F32
-#define NNLBM_CHUNK_REGS_F32 80
+#define NNLBM_CHUNK_REGS_F32 72
 #endif
-// the one-cell cumulant with FP16/BF16 storage gets NNLBM_CHUNK_REGS_CUM16 registers
 #ifndef NNLBM_CHUNK_REGS_CUM16
-#define NNLBM_CHUNK_REGS_CUM16 72
+#define NNLBM_CHUNK_REGS_CUM16 64
 #endif
 template <int DT, int COL, bool PAIR>
 struct StepRegs {
