@@ -623,14 +623,15 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 // continuously, and a few spilled values cost less than the warps that hide the loads; us a step
 // by budget, one B200:
 //   FP32 storage, NNLBM_CHUNK_REGS_F32       72     80     88     96
-//     cumulant, box 192x144x120             151    167    172    174
-//     with mean/rms sums                    195    196    196    205
-//     BGK / MRT_LES, 211x163x137        214/211 226/228 238/230 232/232
+//     cumulant, box 192x144x120             153    157    172    174
+//     with mean/rms sums                    195    193    196    205
+//     junction (CY, sums)                  30.3   29.5
+//     eight junctions                      63.8   61.2
 //   16-bit cumulant, NNLBM_CHUNK_REGS_CUM16  64     72     80     88
-//     box 384x288x240, FP16                 859    881    999   1080
-//   KBC, NNLBM_KBC_REGS                      80     96    104    128
-//     KBC_N4 / N1, FP32 box 176x144x112 183/173 211/200 209/199 208/199
-//     KBC_N4 FP16 junction x0.75           18.5   19.4   19.0   18.7
+//     box 384x288x240, FP16                 842    849    999   1080
+//   KBC, NNLBM_KBC_REGS                      72     80     96    104    128
+//     KBC_N4, FP32 box 176x144x112          206    189    211    209    196
+//     KBC_N4 FP16 junction x0.75           17.8   17.6   19.4   19.0   18.4
 // 16-bit BGK and MRT_LES keep NNLBM_CHUNK_REGS: autotuned, 180.9 to 181.9 us at 64 to 96 on the box
 // of 211x163x137
 #ifndef NNLBM_PAIR_REGS
@@ -643,7 +644,7 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 #define NNLBM_CHUNK_REGS 64
 #endif
 #ifndef NNLBM_CHUNK_REGS_F32
-#define NNLBM_CHUNK_REGS_F32 72
+#define NNLBM_CHUNK_REGS_F32 80
 #endif
 #ifndef NNLBM_CHUNK_REGS_CUM16
 #define NNLBM_CHUNK_REGS_CUM16 64
@@ -675,8 +676,8 @@ struct StepRegs {
 // Addresses come from the plain path's slot bases, the cell's index and the sum of three per-axis
 // wrap offsets (zero for most cells), a reflected direction's from the cell's own slot.  With the
 // wall mask read before the wait for the step before, a halfway junction x0.6 (MRT_LES, every
-// chunk next to a wall) takes 20.3 us a step; with three wrapped coordinates and a 64-bit product
-// for each access, behind the mask's load, it took 24.6
+// chunk next to a wall) takes 19.8 us a step; with three wrapped coordinates and a 64-bit product
+// for each access, behind the mask's load, it took 24.5
 struct WrapOffsets {
     int x[2], y[2], z[2]; // of the neighbours at +1 and -1
     __device__ __forceinline__ WrapOffsets(int c, int yz, int nx, int ny, int nz)
@@ -1140,15 +1141,17 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
     using CT = typename Storage<DT>::CT;
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    // the chunk's record and wall masks, which no step changes, come in while the step before drains
+    // the chunk's record, which no step changes, comes in while the step before drains, and with
+    // halfway walls so do its wall masks.  Elsewhere nothing waits for the record here: a test
+    // of its flags ahead of the wait, with the populations ahead of the control row, cost a
+    // junction (FP32) 1.9 of 30.3 us a step
     constexpr bool pair = PAIR && pairs_chunks(DT, COL);
     Chunk ch{};
     uint32_t hwm = 0u;
+    const bool early = !pair && ODD && ARGS != ARGS_GLOBAL && case_args<ARGS>(g, 0).hw != nullptr;
     if constexpr (!pair) {
-        if (w < g.n_chunks) {
-            ch = g.chunks[w];
-            hwm = chunk_walls<ODD>(case_args<ARGS>(g, ch.cflags & CH_CASE_MASK), ch, lane);
-        }
+        if (w < g.n_chunks) ch = g.chunks[w];
+        if (early) hwm = chunk_walls<ODD>(case_args<ARGS>(g, ch.cflags & CH_CASE_MASK), ch, lane);
     }
     if (g.n_gather == 0) pdl_wait();
     const int step = g.cursor[ODD ? 1 : 0];
@@ -1188,6 +1191,7 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
     } else {
         if (w < g.n_chunks) {
             const int ci = ch.cflags & CH_CASE_MASK;
+            if (!early) hwm = chunk_walls<ODD>(case_args<ARGS>(g, ci), ch, lane);
             fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, hwm, step, flags, lane);
         } else {
             node_batch<DT, ODD>(g.nodes, g.n_nodes, g.cases, g.bc_prof, g.bc_buf, (w - g.n_chunks) * 32 + lane, step, flags);
