@@ -40,7 +40,7 @@ def nvcc() -> str:
 
 def units():
     """(object name, source, extra flags) for every translation unit."""
-    hdrs = [CSRC / "nnlbm_kernels.cuh", CSRC / "nnlbm_physics.cuh", INCLUDE / "nnlbm.h"]
+    hdrs = [CSRC / "nnlbm_kernels.cuh", CSRC / "nnlbm_physics.cuh", CSRC / "nnlbm_physics16.cuh", INCLUDE / "nnlbm.h"]
     out = [("capi", CSRC / "nnlbm_capi.cu", [], hdrs)]
     for dt in range(4):
         prec = F64_FLAGS if dt == 0 else F32_FLAGS

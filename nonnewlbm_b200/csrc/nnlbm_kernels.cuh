@@ -41,7 +41,7 @@
 
 #include <algorithm>
 
-#include "nnlbm_physics.cuh"
+#include "nnlbm_physics16.cuh"
 
 namespace nnlbm {
 
@@ -514,9 +514,10 @@ __device__ __noinline__ void serve_rows(const CaseArgs<typename Storage<DT>::CT>
 }
 
 // called by the whole warp of a chunk with serving lanes (CH_SRC), after its stores; `word` is
-// each lane's word of the node record, rho and u its pre-collision values.  Out of line: inlined
-// it costs the bulk path 7 registers, and with 80 spills
-template <int DT, bool ODD>
+// each lane's word of the node record, rho and u its pre-collision values.  ROWS: the nodes that are
+// lanes of the chunk (CH_ROW) too, where a pair has not written them with its row.  Out of line:
+// inlined it costs the bulk path 7 registers, and with 80 spills
+template <int DT, bool ODD, bool ROWS>
 __device__ __noinline__ void serve_nodes(const CaseArgs<typename Storage<DT>::CT>* ap, const Chunk* chp, unsigned word,
                                          typename Storage<DT>::CT rho, typename Storage<DT>::CT ux, typename Storage<DT>::CT uy,
                                          typename Storage<DT>::CT uz, int step, int flags)
@@ -527,7 +528,15 @@ __device__ __noinline__ void serve_nodes(const CaseArgs<typename Storage<DT>::CT
     const CaseArgs<CT>& a = *ap;
     const NodeWords nw{word};
     const int lane = threadIdx.x & 31, c0 = chp->c0, yz = chp->yz;
-    const unsigned xneg = nw.get(0), xpos = nw.get(1), xreq = nw.get(2), yneg = nw.get(3), ypos = nw.get(4), xeq = nw.get(5);
+    unsigned xneg = nw.get(0), xpos = nw.get(1), xreq = nw.get(2), xeq = nw.get(5);
+    const unsigned yneg = nw.get(3), ypos = nw.get(4);
+    if constexpr (ROWS) {
+        const unsigned l = nw.get(7), r = nw.get(14), eq = nw.get(15);
+        xneg |= l << 1;
+        xpos |= r >> 1;
+        xeq |= (eq & l) << 1;
+        xreq |= (eq & r) >> 1;
+    }
     const int y = yz & 0xffff, z = yz >> 16;
     const int sy = a.nx, x0 = c0 - y * sy - z * sy * a.ny;
     unsigned few = xneg | xpos | yneg | ypos;
@@ -640,6 +649,9 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 #ifndef NNLBM_KBC_REGS
 #define NNLBM_KBC_REGS 80
 #endif
+#ifndef NNLBM_KBC_REGS16
+#define NNLBM_KBC_REGS16 128
+#endif
 #ifndef NNLBM_CHUNK_REGS
 #define NNLBM_CHUNK_REGS 64
 #endif
@@ -647,12 +659,12 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 #define NNLBM_CHUNK_REGS_F32 80
 #endif
 #ifndef NNLBM_CHUNK_REGS_CUM16
-#define NNLBM_CHUNK_REGS_CUM16 64
+#define NNLBM_CHUNK_REGS_CUM16 72
 #endif
 template <int DT, int COL, bool PAIR>
 struct StepRegs {
     static constexpr int value = DT == 0                ? 255
-                                 : !pairs_chunks(DT, COL) ? NNLBM_KBC_REGS
+                                 : !pairs_chunks(DT, COL) ? (DT == 1 ? NNLBM_KBC_REGS : NNLBM_KBC_REGS16)
                                  : PAIR                   ? NNLBM_PAIR_REGS
                                  : DT == 1                ? NNLBM_CHUNK_REGS_F32
                                  : COL == COL_CUM         ? NNLBM_CHUNK_REGS_CUM16
@@ -740,7 +752,7 @@ __device__ __forceinline__ uint32_t chunk_walls(const CaseArgs<CT>& a, const Chu
     return ODD && (ch.cflags & CH_HW) && ((ch.fluid >> lane) & 1u) ? a.hw[ch.c0 + lane] : 0u;
 }
 
-template <int DT, int COL, bool ODD>
+template <int DT, int COL, bool ODD, bool IN_PAIR>
 __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>::CT>& a, const CaseArgs<typename Storage<DT>::CT>* ap,
                                             const Chunk& ch, const Chunk* chp, const ChunkNodes* nodes, uint32_t hwm, int step, int flags,
                                             int lane)
@@ -779,7 +791,7 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
         // one inlined collision for both viscosity models (the local Carreau-Yasuda law is
         // a runtime branch inside it)
         const CYParams<CT> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
-        step_cell<CT, COL, DT, DT != 0, CT>(f, fx, fy, fz, a.nu, a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, a.scale, a.inv_scale,
+        step_cell<CT, COL, DT, DT != 0, ODD, IN_PAIR, CT>(f, fx, fy, fz, a.nu, a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, a.scale, a.inv_scale,
                                             [&](CT r, CT u, CT v, CT w, const CT* Sl) {
             rho = r; ux = u; uy = v; uz = w;
             if ((flags & F_MACRO) || a.cy_mode == CY_REF_FD) {
@@ -826,7 +838,7 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
             }
         }
     }
-    if (ch.cflags & CH_SRC) serve_nodes<DT, ODD>(ap, chp, nw.w, rho, ux, uy, uz, step, flags);
+    if (ch.cflags & CH_SRC) serve_nodes<DT, ODD, false>(ap, chp, nw.w, rho, ux, uy, uz, step, flags);
     if (flags & F_REDUCE) {
         const double s0 = warp_sum(on ? (double)rho : 0.0);
         if (lane == 0 && s0 != 0.0) atomicAdd(red_stripe(a.red, global_warp()), s0);
@@ -1025,7 +1037,7 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
         const int cA = adj ? ca.c0 + 2 * lane : ca.c0 + lane, cB = adj ? ca.c0 + 2 * lane + 1 : cb.c0 + lane;
         const f2 fx(a.fx), fy(a.fy), fz(a.fz);
         const CYParams<float> cy = {a.nu, a.nu0, a.lam, a.a, a.n};
-        step_cell<f2, COL, DT, false, float>(f, fx, fy, fz, f2(a.nu), a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, f2(a.scale),
+        step_cell<f2, COL, DT, false, ODD, true, float>(f, fx, fy, fz, f2(a.nu), a.cy_mode == CY_LOCAL_NEQ ? &cy : nullptr, f2(a.scale),
                                              f2(a.inv_scale), [&](f2 rho, f2 ux, f2 uy, f2 uz, const f2* Sl) {
             r[0] = rho.v.x; r[1] = rho.v.y; u0[0] = ux.v.x; u0[1] = ux.v.y;
             u1[0] = uy.v.x; u1[1] = uy.v.y; u2[0] = uz.v.x; u2[1] = uz.v.y;
@@ -1063,8 +1075,9 @@ __device__ __forceinline__ void pair_finish(const CaseArgs<float>& a, const Case
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const Chunk& ch = h ? cb : ca;
-        if (!(ch.cflags & CH_SRC)) continue;
-        serve_nodes<DT, ODD>(ap, cap + h, ((const unsigned*)(nodes + ch.nodes))[lane & 15], r[h], u0[h], u1[h], u2[h], step, flags);
+        if (!(ch.cflags & (CH_SRC | CH_ROW))) continue;
+        serve_nodes<DT, ODD, (DT >= 2)>(ap, cap + h, ((const unsigned*)(nodes + ch.nodes))[lane & 15], r[h], u0[h], u1[h], u2[h],
+                                        step, flags);
     }
     if (flags & F_REDUCE) {
         const double s0 = warp_sum(mass);
@@ -1088,13 +1101,16 @@ __device__ __forceinline__ void pair_load(const CaseArgs<float>& a, const Chunk&
     }
 }
 
-// two plain chunks of one case (no finite-difference force) collide as a pair
-template <int ARGS>
+// two plain chunks of one case (no finite-difference force) collide as a pair.  With FP32 storage not
+// those with nodes among their own lanes, which leave with the row's stores in the one-cell form.
+// With 16-bit storage those pair too, and the nodes are written after the stores: whether a chunk is
+// one of a pair decides the last bit of what is stored
+template <int DT, int ARGS>
 __device__ __forceinline__ bool pairable(const GroupArgs<float>& g, const Chunk& ca, const Chunk& cb)
 {
     const int ci = ca.cflags & CH_CASE_MASK;
-    return ((ca.cflags & cb.cflags) & CH_PLAIN) && !((ca.cflags | cb.cflags) & CH_ROW) && ci == (cb.cflags & CH_CASE_MASK) &&
-           case_args<ARGS>(g, ci).cy_mode != CY_REF_FD;
+    return ((ca.cflags & cb.cflags) & CH_PLAIN) && (DT >= 2 || !((ca.cflags | cb.cflags) & CH_ROW)) &&
+           ci == (cb.cflags & CH_CASE_MASK) && case_args<ARGS>(g, ci).cy_mode != CY_REF_FD;
 }
 
 // 32 boundary nodes (open-plane nodes and GEO_INFLOW nodes, one per lane): each writes
@@ -1169,19 +1185,19 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
             const Chunk ca = g.chunks[2 * w], cb = g.chunks[2 * w + 1];
             const int ci = ca.cflags & CH_CASE_MASK;
             const CaseArgs<CT>& a = case_args<ARGS>(g, ci);
-            if (pairable<ARGS>(g, ca, cb)) {
+            if (pairable<DT, ARGS>(g, ca, cb)) {
                 f2 f[27];
                 const bool adj = adjacent_span<DT>(ca, cb);
                 if (adj) pair_load_adjacent<DT, ODD>(a, ca.c0, lane, f);
                 else pair_load<DT, ODD>(a, ca, cb, lane, f);
                 pair_finish<DT, COL, ODD>(a, g.cases + ci, ca, cb, g.chunks + 2 * w, g.chunk_nodes, f, step, flags, lane, adj);
             } else {
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
+                fluid_chunk<DT, COL, ODD, true>(a, g.cases + ci, ca, g.chunks + 2 * w, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
                                           flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
                     const CaseArgs<CT>& b = case_args<ARGS>(g, cj);
-                    fluid_chunk<DT, COL, ODD>(b, g.cases + cj, cb, g.chunks + 2 * w + 1, g.chunk_nodes, chunk_walls<ODD>(b, cb, lane),
+                    fluid_chunk<DT, COL, ODD, true>(b, g.cases + cj, cb, g.chunks + 2 * w + 1, g.chunk_nodes, chunk_walls<ODD>(b, cb, lane),
                                               step, flags, lane);
                 }
             }
@@ -1192,7 +1208,7 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
         if (w < g.n_chunks) {
             const int ci = ch.cflags & CH_CASE_MASK;
             if (!early) hwm = chunk_walls<ODD>(case_args<ARGS>(g, ci), ch, lane);
-            fluid_chunk<DT, COL, ODD>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, hwm, step, flags, lane);
+            fluid_chunk<DT, COL, ODD, false>(case_args<ARGS>(g, ci), g.cases + ci, ch, g.chunks + w, g.chunk_nodes, hwm, step, flags, lane);
         } else {
             node_batch<DT, ODD>(g.nodes, g.n_nodes, g.cases, g.bc_prof, g.bc_buf, (w - g.n_chunks) * 32 + lane, step, flags);
         }
@@ -1401,7 +1417,7 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
     auto stage = [&](int u, int b) -> bool {
         if (u >= (g.n_chunks >> 1)) return false;
         const Chunk ca = g.chunks[2 * u], cb = g.chunks[2 * u + 1];
-        if (!pairable<ARGS>(g, ca, cb)) return false;
+        if (!pairable<DT, ARGS>(g, ca, cb)) return false;
         stage_pair<DT, ODD>(case_args<ARGS>(g, ca.cflags & CH_CASE_MASK), ca.c0, cb.c0, lane, buffer(b), &bar[b], g.stage_pad);
         return true;
     };
@@ -1444,12 +1460,12 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
             } else {
                 // inline like the two-cell kernel's, so that both round these chunks alike
                 if (lane == 0) ls[1] = state;
-                fluid_chunk<DT, COL, ODD>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
+                fluid_chunk<DT, COL, ODD, true>(a, g.cases + ci, ca, g.chunks + 2 * u, g.chunk_nodes, chunk_walls<ODD>(a, ca, lane), step,
                                           flags, lane);
                 if (cb.fluid) {
                     const int cj = cb.cflags & CH_CASE_MASK;
                     const CaseArgs<float>& e = case_args<ARGS>(g, cj);
-                    fluid_chunk<DT, COL, ODD>(e, g.cases + cj, cb, g.chunks + 2 * u + 1, g.chunk_nodes, chunk_walls<ODD>(e, cb, lane),
+                    fluid_chunk<DT, COL, ODD, true>(e, g.cases + cj, cb, g.chunks + 2 * u + 1, g.chunk_nodes, chunk_walls<ODD>(e, cb, lane),
                                               step, flags, lane);
                 }
                 __syncwarp();

@@ -227,11 +227,11 @@ __device__ __forceinline__ f2 cy_nu_from_central(f2 Pxx, f2 Pyy, f2 Pzz, f2 Cxy,
 }
 
 // ---------------------------------------------------------------------------------------
-// The collisions work on the stored values themselves: g_q = (f_q - w_q) sc for F32 (sc = 1),
-// FP16 and BF16 storage, f_q for FP64 (DT = 0).  Every moment is linear in them, so the
-// weights and the storage scale meet a handful of moments (or the factors of the equilibrium)
-// instead of each of the 27 populations on the way in and out, and a moment of g carries no
-// rounding of the rest state.  Against populations shifted and scaled one by one, with the
+// The collisions of FP32 and FP64 storage work on the stored values themselves: g_q = f_q - w_q
+// for FP32 (DT = 1), f_q for FP64 (DT = 0).  (Those of the 16-bit types: nnlbm_physics16.cuh.)
+// Every moment is linear in them, so the weights meet a handful of moments (or the factors of
+// the equilibrium) instead of each of the 27 populations on the way in and out, and a moment
+// of g carries no rounding of the rest state.  Against populations shifted and scaled one by one, with the
 // moments summed per use, this halves the instructions of a step.
 //
 // PLANES (one cell in single precision): the planes x = -1 and x = 0 run as f2 pairs on the
@@ -312,28 +312,18 @@ __device__ __forceinline__ Moments<CT> raw_moments(const CT* g)
 }
 
 // what a collision starts from: density (dr = rho - 1 with shifted storage, rho itself with
-// FP64), u = (j + F/2) / rho, its momentum m = j + F/2, the raw moments (in units of f; the
-// second moments on the diagonal less their rest value 1/3 with shifted storage)
+// FP64), u = (j + F/2) / rho, its momentum m = j + F/2, the raw moments (the second moments on
+// the diagonal less their rest value 1/3 with shifted storage)
 template <class CT>
 struct CellState {
     Moments<CT> M;
     CT dr, rho, ir, mx, my, mz, ux, uy, uz;
 };
-template <class CT, int DT, bool PLANES, bool THIRD>
-__device__ __forceinline__ CellState<CT> cell_state(const CT* g, CT fx, CT fy, CT fz, CT isc)
+template <class CT, int DT, bool PLANES>
+__device__ __forceinline__ CellState<CT> cell_state(const CT* g, CT fx, CT fy, CT fz)
 {
     CellState<CT> c;
     c.M = raw_moments<CT, PLANES>(g);
-    if constexpr (DT >= 2) {
-        Moments<CT>& M = c.M;
-        M.r = M.r * isc; M.jx = M.jx * isc; M.jy = M.jy * isc; M.jz = M.jz * isc;
-        M.xx = M.xx * isc; M.yy = M.yy * isc; M.zz = M.zz * isc;
-        M.xy = M.xy * isc; M.xz = M.xz * isc; M.yz = M.yz * isc;
-        if constexpr (THIRD) {
-            M.xxy = M.xxy * isc; M.xxz = M.xxz * isc; M.xyy = M.xyy * isc; M.yyz = M.yyz * isc;
-            M.xzz = M.xzz * isc; M.yzz = M.yzz * isc; M.xyz = M.xyz * isc;
-        }
-    }
     c.dr = c.M.r;
     c.rho = DT == 0 ? c.dr : c.dr + CT(1);
     c.ir = CT(1) / c.rho;
@@ -396,26 +386,25 @@ __device__ __forceinline__ void to_pops(V& a, V& b, V& c)
     c = p;
 }
 
-// scaled central moments of a cell after the collision, times the storage scale: the halves
-// and quarters of the second order (x = s200/2, a = s110/4, ...) and the density
+// scaled central moments of a cell after the collision: the halves and quarters of the second order (x = s200/2, a = s110/4, ...) and the density
 template <class CT>
 struct CumPost { CT r, x, y, z, a, b, c; };  // a: 110, b: 101, c: 011
 
 // the raw moments k[i][j][l] of the post-collision state (x pass; the orders that vanish are
 // left out of the arithmetic)
 template <class CT>
-__device__ __forceinline__ void cum_x_raw(const CumPost<CT>& s, CT irs, CT ux, CT fx, CT fy, CT fz, CT (&k)[3][3][3])
+__device__ __forceinline__ void cum_x_raw(const CumPost<CT>& s, CT ir, CT ux, CT fx, CT fy, CT fz, CT (&k)[3][3][3])
 {
     const CT uh = CT(0.5) * ux;
     const CT four = CT(4), eight = CT(8);
     // fourth and sixth order from products
-    const CT s211 = mad(s.x, s.c, four * (s.a * s.b)) * irs;
-    const CT s121 = mad(s.y, s.b, four * (s.a * s.c)) * irs;
-    const CT s112 = mad(s.z, s.a, four * (s.b * s.c)) * irs;
-    const CT s220 = mad(s.x, s.y, eight * (s.a * s.a)) * irs;
-    const CT s202 = mad(s.x, s.z, eight * (s.b * s.b)) * irs;
-    const CT s022 = mad(s.y, s.z, eight * (s.c * s.c)) * irs;
-    const CT s222 = mad(s.x, s022, eight * mad(s.b, s121, s.a * s112)) * irs;
+    const CT s211 = mad(s.x, s.c, four * (s.a * s.b)) * ir;
+    const CT s121 = mad(s.y, s.b, four * (s.a * s.c)) * ir;
+    const CT s112 = mad(s.z, s.a, four * (s.b * s.c)) * ir;
+    const CT s220 = mad(s.x, s.y, eight * (s.a * s.a)) * ir;
+    const CT s202 = mad(s.x, s.z, eight * (s.b * s.b)) * ir;
+    const CT s022 = mad(s.y, s.z, eight * (s.c * s.c)) * ir;
+    const CT s222 = mad(s.x, s022, eight * mad(s.b, s121, s.a * s112)) * ir;
     // first order F/2 (times 1/2)
     k[0][0][0] = s.r; k[1][0][0] = CT(0.25) * fx; k[2][0][0] = s.x;
     to_raw<CT>(ux, uh, k[0][0][0], k[1][0][0], k[2][0][0]);
@@ -442,18 +431,15 @@ __device__ __forceinline__ void cum_x_raw(const CumPost<CT>& s, CT irs, CT ux, C
 }
 
 template <class CT, int DT, bool PLANES>
-__device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, const Central<CT>& C, CT fx, CT fy, CT fz, CT nu, CT sc,
-                                            CT isc)
+__device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, const Central<CT>& C, CT fx, CT fy, CT fz, CT nu)
 {
     const CT om = CT(1) / (CT(3) * nu + CT(0.5));
     // relaxation (lbm_col_cum.h:205-235 with omega2 = 1): the shear parts by omega1, the trace
-    // to rho; all times the storage scale
-    const CT k = DT >= 2 ? (CT(1) - om) * sc : CT(1) - om;
-    const CT irs = DT >= 2 ? c.ir * isc : c.ir;
-    if constexpr (DT >= 2) { fx = fx * sc; fy = fy * sc; fz = fz * sc; }
+    // to rho
+    const CT k = CT(1) - om;
     const CT e1 = k * (C.xx - C.yy), e2 = k * (C.xx - C.zz), kq = CT(0.25) * k;
     CumPost<CT> s;
-    s.r = DT >= 2 ? c.rho * sc : c.rho;
+    s.r = c.rho;
     s.x = CT(1.0 / 6.0) * ((e1 + e2) + s.r);
     s.y = mad(CT(-0.5), e1, s.x);
     s.z = mad(CT(-0.5), e2, s.x);
@@ -461,11 +447,11 @@ __device__ __forceinline__ void collide_cum(CT* g, const CellState<CT>& c, const
     s.b = kq * C.xz;
     s.c = kq * C.yz;
     CT m[3][3][3];
-    cum_x_raw<CT>(s, irs, c.ux, fx, fy, fz, m);
-    const CT w1 = DT >= 2 ? sc * CT(1.0 / 6.0) : CT(1.0 / 6.0);
+    cum_x_raw<CT>(s, c.ir, c.ux, fx, fy, fz, m);
+    const CT w1 = CT(1.0 / 6.0);
     const CT w2 = w1 * CT(1.0 / 6.0), w3 = w2 * CT(1.0 / 6.0);
     // the rest state's raw moments (times 1/2 per axis of order 2) off plane m[i] (order i in x)
-    const CT r0 = DT >= 2 ? c.dr * sc : c.dr;
+    const CT r0 = c.dr;
     if constexpr (PLANES) {
         // orders i = 0, 1 in x as pairs, i = 2 scalar
         f2 P[3][3];
@@ -565,25 +551,25 @@ __device__ __forceinline__ bool any_force(f2 fx, f2 fy, f2 fz)
 {
     return any_force(fx.v.x, fy.v.x, fz.v.x) || any_force(fx.v.y, fy.v.y, fz.v.y);
 }
-// g_q += k S_q feq_q sc for every direction (rs = rho sc), out of line on a copy, so that the
+// g_q += k S_q feq_q for every direction, out of line on a copy, so that the
 // path without a force keeps its populations in registers
 template <class CT>
-__device__ __noinline__ void add_force_all(CT* g, CT k, CT rs, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
+__device__ __noinline__ void add_force_all(CT* g, CT k, CT rho, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
 {
     const FactEq<CT> E(ux, uy, uz);
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
-        const CT feq = -rs * E.X[q / 9] * E.Y[(q / 3) % 3] * E.Z[q % 3];
+        const CT feq = -rho * E.X[q / 9] * E.Y[(q / 3) % 3] * E.Z[q % 3];
         g[q] += k * force_src<CT>(q, ir, ux, uy, uz, fx, fy, fz) * feq;
     }
 }
 template <class CT>
-__device__ __forceinline__ void add_force(CT* g, CT k, CT rs, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
+__device__ __forceinline__ void add_force(CT* g, CT k, CT rho, CT ir, CT ux, CT uy, CT uz, CT fx, CT fy, CT fz)
 {
     CT t[27];
 #pragma unroll
     for (int q = 0; q < 27; ++q) t[q] = g[q];
-    add_force_all<CT>(t, k, rs, ir, ux, uy, uz, fx, fy, fz);
+    add_force_all<CT>(t, k, rho, ir, ux, uy, uz, fx, fy, fz);
 #pragma unroll
     for (int q = 0; q < 27; ++q) g[q] = t[q];
 }
@@ -646,12 +632,11 @@ struct GridEq {
 // BGK, solver/lbm3d/lbm_col_bgk.h:14-140: g' = (1 - om) g + om geq, the factor om inside geq:
 // two operations a direction
 template <class CT, int DT, bool PLANES>
-__device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, CT sc)
+__device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu)
 {
     const CT om = CT(1) / (CT(3) * nu + CT(0.5));
-    const CT rs = DT >= 2 ? c.rho * sc : c.rho, drs = DT >= 2 ? c.dr * sc : c.dr;
     CT Fx[3], Fy[3], Fz[3];
-    const GridEq<CT, DT> E(c.ux, c.uy, c.uz, om * rs, om * drs, Fx, Fy, Fz);
+    const GridEq<CT, DT> E(c.ux, c.uy, c.uz, om * c.rho, om * c.dr, Fx, Fy, Fz);
     const CT k = CT(1) - om;
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -668,7 +653,7 @@ __device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx
             }
             g[18 + q] = mad(k, g[18 + q], E(2, j, l));
         }
-    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - CT(0.5) * om, rs, c.ir, c.ux, c.uy, c.uz, fx, fy, fz);
+    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - CT(0.5) * om, c.rho, c.ir, c.ux, c.uy, c.uz, fx, fy, fz);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -678,7 +663,7 @@ __device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx
 // share their even part and differ by the sign of the odd one (3 rho c.u).
 // ---------------------------------------------------------------------------------------
 template <class CT, int DT>
-__device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu, CT sc)
+__device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu)
 {
     const Moments<CT>& M = c.M;
     const CT third = c.dr * CT(1.0 / 3.0);
@@ -688,14 +673,13 @@ __device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu
     const CT tau = CT(3) * nu + CT(0.5);
     const CT om = CT(2) / (dsqrt<CT>(tau * tau + CT(2) * CT(0.0342) * CT(9) * dsqrt<CT>(Qs) * c.ir) + tau);
     const CT Pxx = mad(-om, nxx, M.xx), Pyy = mad(-om, nyy, M.yy), Pzz = mad(-om, nzz, M.zz);
-    const CT sn = DT >= 2 ? CT(9) * sc : CT(9);
+    const CT sn = CT(9);
     const CT xy = sn * mad(-om, nxy, M.xy), xz = sn * mad(-om, nxz, M.xz), yz = sn * mad(-om, nyz, M.yz);
-    const CT s1 = DT >= 2 ? sc : CT(1);
     // even part: A + B_a per axis with c_a != 0 + 9 c_a c_b P_ab; odd part: 3 rho c.u
-    const CT h = s1 * CT(1.5);
-    const CT A = DT >= 2 ? s1 * mad(CT(-1.5), (Pxx + Pyy) + Pzz, CT(2.5) * c.dr) : mad(CT(-1.5), (Pxx + Pyy) + Pzz, CT(2.5) * c.dr);
+    const CT h = CT(1.5);
+    const CT A = mad(CT(-1.5), (Pxx + Pyy) + Pzz, CT(2.5) * c.dr);
     const CT bx = h * mad(CT(3), Pxx, -c.dr), by = h * mad(CT(3), Pyy, -c.dr), bz = h * mad(CT(3), Pzz, -c.dr);
-    const CT s3 = s1 * CT(3);
+    const CT s3 = CT(3);
     const CT jx = s3 * c.mx, jy = s3 * c.my, jz = s3 * c.mz;
     // direction q and its opposite from the even and odd parts
     auto put = [&](int q, CT e, CT o) {
@@ -723,7 +707,7 @@ __device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu
 // ds = s(m) - s(m_eq) = s(m - m_eq).  The 27 ds are formed once (opposite directions share
 // their even part) and serve both passes: the products of the stabiliser, whose 1/feq is
 // the product of the inverse factors, and the relaxation
-// g' = g - beta gamma (g - geq) - beta (2 - gamma) ds, geq = (feq - w) sc.
+// g' = g - beta gamma (g - geq) - beta (2 - gamma) ds, geq = feq - w.
 // ---------------------------------------------------------------------------------------
 // the entropic stabiliser gamma = 1/beta - (2 - 1/beta) num/den; the reference divides 0/0
 // when dh vanishes identically, where gamma*dh is zero for any finite gamma and the
@@ -735,7 +719,7 @@ __device__ __forceinline__ CT kbc_gamma(CT num, CT den, CT beta)
 }
 
 // ds_q of the moment differences: trace T, normal differences Nxz, Nyz, shears P, third order
-// (its order: xxy xxz xyy yyz xzz yzz xyz), times the storage scale
+// (its order: xxy xxz xyy yyz xzz yzz xyz)
 template <class CT, bool USE_T, bool USE_Q>
 __device__ __forceinline__ void kbc_shear(CT T, CT Nxz, CT Nyz, CT Pxy, CT Pxz, CT Pyz, const CT* Q, CT* ds)
 {
@@ -768,7 +752,7 @@ __device__ __forceinline__ void kbc_shear(CT T, CT Nxz, CT Nyz, CT Pxy, CT Pxz, 
 }
 
 template <class CT, int DT, bool CENTRAL, bool USE_T, bool USE_Q>
-__device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu, CT sc)
+__device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx, CT fy, CT fz, CT nu)
 {
     const Moments<CT>& M = c.M;
     const CT rho = c.rho, ux = c.ux, uy = c.uy, uz = c.uz;
@@ -800,17 +784,11 @@ __device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx
         Q[5] = M.yzz - cs2 * (s * uz * Pyz + uy * (three * zz - Nyz - Nxz + cT));
         Q[6] = M.xyz - ux * Pyz - uy * Pxz - uz * Pxy - ux * uy * uz;
     }
-    if constexpr (DT >= 2) {
-        T = T * sc; Nxz = Nxz * sc; Nyz = Nyz * sc; Pxy = Pxy * sc; Pxz = Pxz * sc; Pyz = Pyz * sc;
-#pragma unroll
-        for (int i = 0; i < 7; ++i) Q[i] = Q[i] * sc;
-    }
     CT ds[27];
     kbc_shear<CT, USE_T, USE_Q>(T, Nxz, Nyz, Pxy, Pxz, Pyz, Q, ds);
     const CT beta = CT(1) / (CT(6) * nu + CT(1));
-    const CT rs = DT >= 2 ? rho * sc : rho, drs = DT >= 2 ? c.dr * sc : c.dr;
     CT Fx[3], Fy[3], Fz[3];
-    const GridEq<CT, DT> E(ux, uy, uz, rs, drs, Fx, Fy, Fz);
+    const GridEq<CT, DT> E(ux, uy, uz, rho, c.dr, Fx, Fy, Fz);
     CT num = CT(0), den = CT(0);
     {
         const CT iZ[3] = {CT(1) / Fz[0], CT(1) / Fz[1], CT(1) / Fz[2]};
@@ -840,19 +818,15 @@ __device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx
                 const int q = 9 * i + 3 * j + l;
                 g[q] = mad(-b2, ds[q], mad(-bg, g[q] - E(i, j, l), g[q]));
             }
-    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - beta, rs, c.ir, ux, uy, uz, fx, fy, fz);
+    if (any_force(fx, fy, fz)) add_force<CT>(g, CT(1) - beta, rho, c.ir, ux, uy, uz, fx, fy, fz);
 }
 
-// density, velocity (u = (j + F/2) / rho) and the collision of one cell's stored values g (or
-// of two cells', CT = f2).  With `cy` the shear viscosity is the local Carreau-Yasuda one.  PT: the
-// type of the viscosity-law parameters.  out(rho, ux, uy, uz, S) is called once they are known
-// (S: the strain rate with `cy`, else null), before the populations are rebuilt, so that
-// nothing of it is held in registers meanwhile
+// density, velocity and collision of one cell's stored values (or of two cells', CT = f2) with FP32 or
+// FP64 storage; see step_cell in nnlbm_physics16.cuh
 template <class CT, int COL, int DT, bool PLANES, class PT, class Out>
-__device__ __forceinline__ void step_cell(CT* g, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, CT sc, CT isc, Out&& out)
+__device__ __forceinline__ void step_cell_stored(CT* g, CT fx, CT fy, CT fz, CT nu, const CYParams<PT>* cy, Out&& out)
 {
-    constexpr bool KBC = COL >= COL_KBC_N1 && COL <= COL_KBC_C4;
-    const CellState<CT> c = cell_state<CT, DT, PLANES, KBC>(g, fx, fy, fz, isc);
+    const CellState<CT> c = cell_state<CT, DT, PLANES>(g, fx, fy, fz);
     Central<CT> C;
     if (COL == COL_CUM || cy) C = central_moments<CT>(c, fx, fy, fz);
     if (cy) {
@@ -863,15 +837,15 @@ __device__ __forceinline__ void step_cell(CT* g, CT fx, CT fy, CT fz, CT nu, con
         out(c.rho, c.ux, c.uy, c.uz, (const CT*)nullptr);
     }
     if constexpr (COL == COL_CUM) {
-        collide_cum<CT, DT, PLANES>(g, c, C, fx, fy, fz, nu, sc, isc);
+        collide_cum<CT, DT, PLANES>(g, c, C, fx, fy, fz, nu);
     } else if constexpr (COL == COL_MRT) {
-        collide_mrt<CT, DT>(g, c, nu, sc);
+        collide_mrt<CT, DT>(g, c, nu);
     } else if constexpr (COL == COL_BGK) {
-        collide_bgk<CT, DT, PLANES>(g, c, fx, fy, fz, nu, sc);
+        collide_bgk<CT, DT, PLANES>(g, c, fx, fy, fz, nu);
     } else {
         constexpr bool central = COL >= COL_KBC_C1;
         constexpr int v = central ? COL - COL_KBC_C1 + 1 : COL - COL_KBC_N1 + 1;
-        collide_kbc<CT, DT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(g, c, fx, fy, fz, nu, sc);
+        collide_kbc<CT, DT, central, (v == 2 || v == 4), (v == 3 || v == 4)>(g, c, fx, fy, fz, nu);
     }
 }
 
