@@ -540,15 +540,16 @@ __device__ __noinline__ void serve_nodes(const CaseArgs<typename Storage<DT>::CT
     const int y = yz & 0xffff, z = yz >> 16;
     const int sy = a.nx, x0 = c0 - y * sy - z * sy * a.ny;
     unsigned few = xneg | xpos | yneg | ypos;
-    if (__popc(few & ~xeq) > 4) {
+    const bool rows = __popc(few & ~xeq) > 4;
+    if (rows) {
         const unsigned bit = 1u << lane;
         const unsigned dirs = ((xneg & ~xeq & bit) ? 1u : 0u) | ((xpos & bit) ? 2u : 0u) | ((yneg & bit) ? 4u : 0u) |
                               ((ypos & bit) ? 8u : 0u);
         if (dirs) serve_rows<DT, ODD>(ap, c0 + lane, x0 + lane, y, z, dirs, (xreq & bit) != 0, rho, ux, uy, uz, step, flags);
         few = xeq; // the GEO_INFLOW node is left, which the whole warp writes
     }
-    // few serving lanes: the warp writes each node, lane q population q
-    const bool rows = few == xeq;
+    // few serving lanes (or the GEO_INFLOW node after serve_rows wrote the others): the warp writes each
+    // node, lane q population q
     for (unsigned todo = few; todo; todo &= todo - 1) {
         const int s = __ffs(todo) - 1;
         const CT rs = __shfl_sync(0xffffffffu, rho, s), us = __shfl_sync(0xffffffffu, ux, s);
