@@ -575,47 +575,66 @@ __device__ __forceinline__ void add_force(CT* g, CT k, CT rho, CT ir, CT ux, CT 
 }
 
 // The equilibrium of BGK and KBC in the units of the stored values, geq_q = (feq_q - w_q) s
-// (feq_q s with FP64 storage).  Per axis the factor is its weight W (1/6, 2/3, 1/6) plus a
+// (feq_q s with FP64 storage).  Per axis the factor F is its weight W (1/6, 2/3, 1/6) plus a
 // deviation A ((u^2 - u)/2, -u^2, (u^2 + u)/2); the product less w_q is collected as
-//   X_i b_jl + T_i,n,   b_jl = A_j F_l + W_j A_l,  F = W + A,  X_i = s rho F_i,
-//   T_i,n = (s rho A_i + s (rho - 1) W_i) W_j W_l
+//   F_i b_jl + T_i,n,   b_jl = B_j F_l + W_j B_l,  B = s rho A,
+//   T_i,n = (B_i + s (rho - 1) W_i) W_j W_l
 // so that nothing of the size of w_q is ever rounded and taken off again (a population's
-// error would then be a bias of the density, the same in every step)
+// error would then be a bias of the density, the same in every step).
+//
+// The rounded constants would be such a bias too: the sums over an axis have to be exact, sum F = 1,
+// F_+ - F_- = u, sum W = 1, T_0 + 4 T_1 + 4 T_2 = B_i + s (rho - 1) W_i.  So W and the products of
+// two W are floats that add up (each within 1.2 units of its value), and with FP64 the outer F come from
+// the middle one.  And so would rho u in place of the momentum m, since 1/rho just above 1 rounds up
+// more often than down: B = s (m u - m)/2, -s m u, s (m u + m)/2.  Change per step on a periodic lattice
+// (24x20x16 cells, 3000 steps), with constants and rho u rounded by themselves -> now: FP64 mass
+// 3.3e-16 -> 4e-20 a cell, FP32 momentum (BGK, KBC_N4) 1.3e-7 -> 1.4e-9, 1.2e-9 of it
 template <class CT, int DT>
 struct GridEq {
     CT X[3], T[3][3], b[3][3];
-    __device__ static __forceinline__ void axis(CT u, CT* A, CT* F)
+    // 1/6 and 2/3 as floats with 2 W0 + W1 = 1
+    static constexpr double W0 = 11184810.0 / 67108864.0, W1 = 11184811.0 / 16777216.0;
+    // p = s m / 2
+    __device__ static __forceinline__ void axis(CT u, CT p, CT* B, CT* F)
     {
-        const CT h = CT(0.5) * u, uu = u * u;
-        A[1] = -uu;
-        A[2] = mad(h, u, h);
-        A[0] = mad(h, u, -h);
+        B[1] = CT(-2) * p * u;
+        B[2] = mad(p, u, p);
+        B[0] = mad(p, u, -p);
+        const CT uu = u * u;
         F[1] = CT(2.0 / 3.0) - uu;
-        F[2] = CT(1.0 / 6.0) + A[2];
-        F[0] = CT(1.0 / 6.0) + A[0];
+        if constexpr (DT == 0) {
+            F[2] = CT(0.5) * ((CT(1) - F[1]) + u);
+            F[0] = F[2] - u;
+        } else {
+            const CT e = mad(CT(0.5), uu, CT(W0));
+            F[2] = mad(CT(0.5), u, e);
+            F[0] = mad(CT(-0.5), u, e);
+        }
     }
-    // s rho, s (rho - 1)
-    __device__ __forceinline__ GridEq(CT ux, CT uy, CT uz, CT rs, CT drs, CT* Fx, CT* Fy, CT* Fz)
+    __device__ __forceinline__ GridEq(const CellState<CT>& c, CT s, CT* Fx, CT* Fy, CT* Fz)
     {
-        CT Ax[3], Ay[3], Az[3];
-        axis(ux, Ax, Fx);
-        axis(uy, Ay, Fy);
-        axis(uz, Az, Fz);
-        const CT W[3] = {CT(1.0 / 6.0), CT(2.0 / 3.0), CT(1.0 / 6.0)};
+        const CT h = CT(0.5) * s;
+        CT Bx[3], By[3], Bz[3];
+        axis(c.ux, h * c.mx, Bx, Fx);
+        axis(c.uy, h * c.my, By, Fy);
+        axis(c.uz, h * c.mz, Bz, Fz);
+        const CT W[3] = {CT(W0), CT(W1), CT(W0)};
+        const CT sr = s * c.rho, sd = s * c.dr;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            X[i] = rs * Fx[i];
+            X[i] = DT == 0 ? sr * Fx[i] : Fx[i];
             if constexpr (DT != 0) {
-                const CT t = mad(rs, Ax[i], drs * W[i]);
-                T[i][0] = t * CT(4.0 / 9.0);
-                T[i][1] = t * CT(1.0 / 9.0);
-                T[i][2] = t * CT(1.0 / 36.0);
+                const CT t = mad(sd, W[i], Bx[i]);
+                // 4/9, 1/9, 1/36 as floats with K_0 + 4 K_1 + 4 K_2 = 1
+                T[i][0] = t * CT(14913082.0 / 33554432.0);
+                T[i][1] = t * CT(14913080.0 / 134217728.0);
+                T[i][2] = t * CT(14913080.0 / 536870912.0);
             }
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j)
 #pragma unroll
-            for (int l = 0; l < 3; ++l) b[j][l] = DT == 0 ? Fy[j] * Fz[l] : mad(Ay[j], Fz[l], W[j] * Az[l]);
+            for (int l = 0; l < 3; ++l) b[j][l] = DT == 0 ? Fy[j] * Fz[l] : mad(By[j], Fz[l], W[j] * Bz[l]);
     }
     __device__ __forceinline__ CT operator()(int i, int j, int l) const
     {
@@ -636,7 +655,7 @@ __device__ __forceinline__ void collide_bgk(CT* g, const CellState<CT>& c, CT fx
 {
     const CT om = CT(1) / (CT(3) * nu + CT(0.5));
     CT Fx[3], Fy[3], Fz[3];
-    const GridEq<CT, DT> E(c.ux, c.uy, c.uz, om * c.rho, om * c.dr, Fx, Fy, Fz);
+    const GridEq<CT, DT> E(c, om, Fx, Fy, Fz);
     const CT k = CT(1) - om;
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -687,10 +706,19 @@ __device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu
         g[q] = w * (e + o);
         g[26 - q] = w * (e - o);
     };
-    g[13] = CT(weight<double>(13)) * A;
     const CT ax = A + bx, ay = A + by, az = A + bz;
-    put(22, ax, jx); put(16, ay, jy); put(14, az, jz);
+    // The rounded weights all carry the same factor 1 + 5e-9 (FP32), which would be a bias of what is
+    // conserved: along an axis the odd part is what the others leave of the momentum,
+    // m/2 - 4 (w_25 + w_26) j, and the rest population what they leave of the density
+    auto axis = [&](int q, CT e, CT m, CT j) {
+        const CT o = mad(CT(-5), CT(weight<double>(25)) * j, CT(0.5) * m);
+        const CT w = CT(weight<double>(q));
+        g[q] = mad(w, e, o);
+        g[26 - q] = mad(w, e, -o);
+    };
+    axis(22, ax, c.mx, jx); axis(16, ay, c.my, jy); axis(14, az, c.mz, jz);
     const CT axy = ax + by, axz = ax + bz, ayz = ay + bz, all = axy + bz;
+    g[13] = mad(-CT(weight<double>(22)), mad(CT(2), (ax + ay) + az, mad(CT(0.5), all, (axy + axz) + ayz)), c.dr);
     put(25, axy + xy, jx + jy); put(19, axy - xy, jx - jy);
     put(23, axz + xz, jx + jz); put(21, axz - xz, jx - jz);
     put(17, ayz + yz, jy + jz); put(15, ayz - yz, jy - jz);
@@ -788,9 +816,10 @@ __device__ __forceinline__ void collide_kbc(CT* g, const CellState<CT>& c, CT fx
     kbc_shear<CT, USE_T, USE_Q>(T, Nxz, Nyz, Pxy, Pxz, Pyz, Q, ds);
     const CT beta = CT(1) / (CT(6) * nu + CT(1));
     CT Fx[3], Fy[3], Fz[3];
-    const GridEq<CT, DT> E(ux, uy, uz, rho, c.dr, Fx, Fy, Fz);
+    const GridEq<CT, DT> E(c, CT(1), Fx, Fy, Fz);
     CT num = CT(0), den = CT(0);
     {
+        // 1/feq, less the factor rho with FP32 storage (gamma takes the ratio of the sums)
         const CT iZ[3] = {CT(1) / Fz[0], CT(1) / Fz[1], CT(1) / Fz[2]};
 #pragma unroll
         for (int i = 0; i < 3; ++i)
