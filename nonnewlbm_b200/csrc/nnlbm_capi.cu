@@ -546,8 +546,8 @@ bool can_stage(const nnlbm_ctx* ctx, const Group& g)
 }
 
 // the kernels of one step with the group arguments `args` (no host synchronisation); `odd` is
-// the A-A parity.  `chained`: each kernel as a programmatic dependent of the one before it;
-// `only_step`: without the kernels before the step kernel itself
+// the A-A parity.  `chained`: each kernel but the gather as a programmatic dependent of the one
+// before it; `only_step`: without the kernels before the step kernel itself
 int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool odd, bool chained, bool only_step = false)
 {
     const AuxLaunchers& A = aux_launchers(g.dtype);
@@ -558,7 +558,7 @@ int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool o
         A.refd_velocity(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
         A.refd_stress(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
     }
-    if (!only_step && g.n_gather > 0) A.gather(odd, chained, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
+    if (!only_step && g.n_gather > 0) A.gather(odd, false, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     dim3 grid = blocks(step_warps(g), per_block), block(g.block);
     int form = g.paired ? FORM_PAIRED : FORM_ONE;
     if (g.staged) {

@@ -225,13 +225,18 @@ __host__ __device__ constexpr int args_mode(int n_cases)
 // that the launch of each overlaps the end of the one before.  A step launches the open-plane
 // gather, where it has nodes to gather, and the step kernel; with the finite-difference
 // Carreau-Yasuda coupling its velocity and strain kernels first, each waiting for the one before.
-//   - The first kernel of a step waits for the step before as its first act.
-//   - The gather then lets the step kernel start at once.  The slots that it reads are
-//     overwritten by the step: the chunks that hold them (CH_WAIT) and the node warps wait for
-//     it before their first store.  The step kernel itself leaves the next kernel's start to
-//     its own end: with an earlier trigger the next step's blocks come up while this one's are
-//     running, and measured slower (pipe 96x32x32 7.5 us a step against 6.5, junction 31.2
-//     against 30.1).
+//   - A chained kernel waits for the one before ahead of everything that a step changes; only work-list
+//     records, wall masks and labels are read earlier.
+//   - The gather is not chained: it starts once the kernel before it has ended, and lets the step kernel
+//     start at once, which so sees all that the kernels before the gather wrote without a wait of its
+//     own (a wait in the gather alone would order nothing for the step kernel).  The slots that
+//     the gather reads are overwritten by the step: the chunks that hold them (CH_WAIT) and the node
+//     warps wait for it before their first store.  us a step, gather chained -> not: FP32 box
+//     192x144x120 158.9 -> 153.0, KBC_N4 box 192.3 -> 185.2, ref-fd junction x0.5 28.7 -> 29.0; with a
+//     step kernel that waits for the gather first 162.9, 197.4, 32.5.
+//   - The step kernel itself leaves the next kernel's start to its own end: with an earlier trigger
+//     the next step's blocks come up while this one's are running, and measured slower (pipe
+//     96x32x32 7.5 us a step against 6.5, junction 31.2 against 30.1).
 //   - Every kernel waits before it ends, so that its completion implies that of the kernels
 //     before it, which is all the next step waits for.
 // Where a kernel is launched without the attribute the waits return at once.
@@ -1531,7 +1536,6 @@ template <int DT, bool ODD, int ARGS>
 __global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupArgs<typename Storage<DT>::CT> g)
 {
     using CT = typename Storage<DT>::CT;
-    pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.n_gather) return;

@@ -707,7 +707,7 @@ __device__ __forceinline__ void collide_mrt(CT* g, const CellState<CT>& c, CT nu
         g[26 - q] = w * (e - o);
     };
     const CT ax = A + bx, ay = A + by, az = A + bz;
-    // The rounded weights all carry the same factor 1 + 5e-9 (FP32), which would be a bias of what is
+    // The rounded weights all carry the same factor 1 + 7.6e-9 (FP32), which would be a bias of what is
     // conserved: along an axis the odd part is what the others leave of the momentum,
     // m/2 - 4 (w_25 + w_26) j, and the rest population what they leave of the density
     auto axis = [&](int q, CT e, CT m, CT j) {
