@@ -1452,7 +1452,7 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
                     if (lane == 0) atomicOr(a.err, ERR_STALL);
                     // the copies of the next pair are this warp's: let them land before it leaves
                     if (state & 2) mbar_wait(&bar[b ^ 1], (state >> (3 - b)) & 1, g.stage_wait_ns);
-                    return;
+                    break; // to the wait that every kernel of a step ends with
                 }
                 state ^= 4 << b;
                 // the loop state waits in shared memory while the pair collides
