@@ -572,30 +572,35 @@ int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool o
     return NNLBM_OK;
 }
 
-// kChainSteps steps of either starting parity as one CUDA graph: inside it the kernels follow one
+// kChainSteps steps from parity p as one CUDA graph, made when a call first needs it (an even number, so
+// that a call launches the graph of its own starting parity only): inside it the kernels follow one
 // another programmatically at 1.1-1.4 us a kernel, where one graph or kernel launch per step puts
 // 2-4 us between two steps (measured with empty kernels of 148 and 1000 blocks).  Shorter calls,
 // and the steps left over, are launched one by one, chained too: a call of a few steps pays for
 // no capture
 constexpr int kChainSteps = 16;
-int ensure_graphs(nnlbm_ctx* ctx, Group& g)
+static_assert(kChainSteps % 2 == 0, "a graph leaves the parity that it starts from");
+int ensure_graph(nnlbm_ctx* ctx, Group& g, int p)
 {
-    if (g.graph[0] && g.graph[1] && g.graph_gen == g.gen) return NNLBM_OK;
-    for (int p = 0; p < 2; ++p) {
-        if (g.graph[p]) { cudaGraphExecDestroy(g.graph[p]); g.graph[p] = nullptr; }
-        cudaGraph_t gr = nullptr;
-        CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = NNLBM_OK;
-        for (int k = 0; k < kChainSteps && rc == NNLBM_OK; ++k)
-            rc = launch_step_kernels(ctx, g, g.args.data(), ((p + k) & 1) != 0, true);
-        cudaError_t e = cudaStreamEndCapture(ctx->stream, &gr);
-        if (rc != NNLBM_OK) { if (gr) cudaGraphDestroy(gr); return rc; }
-        if (e != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&g.graph[p], gr, 0);
-        cudaGraphDestroy(gr);
-        if (e != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
+    if (g.graph_gen != g.gen) {
+        for (cudaGraphExec_t& e : g.graph) {
+            if (e) cudaGraphExecDestroy(e);
+            e = nullptr;
+        }
+        g.graph_gen = g.gen;
     }
-    g.graph_gen = g.gen;
+    if (g.graph[p]) return NNLBM_OK;
+    cudaGraph_t gr = nullptr;
+    CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = NNLBM_OK;
+    for (int k = 0; k < kChainSteps && rc == NNLBM_OK; ++k)
+        rc = launch_step_kernels(ctx, g, g.args.data(), ((p + k) & 1) != 0, true);
+    cudaError_t e = cudaStreamEndCapture(ctx->stream, &gr);
+    if (rc != NNLBM_OK) { if (gr) cudaGraphDestroy(gr); return rc; }
+    if (e != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+    e = cudaGraphInstantiate(&g.graph[p], gr, 0);
+    cudaGraphDestroy(gr);
+    if (e != cudaSuccess) return set_err(ctx, NNLBM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
     return NNLBM_OK;
 }
 
@@ -712,8 +717,8 @@ int run_group_steps(nnlbm_ctx* ctx, Group& g, int64_t n, int flags, bool use_gra
     int rc = prepare_steps(ctx, g, n, flags, reset);
     if (rc) return rc;
     use_graph = use_graph && n >= 2 * kChainSteps;
-    if (use_graph && (rc = ensure_graphs(ctx, g)) != NNLBM_OK) return rc;
     const int64_t parity = ctx->cases[g.cases[0]].parity;
+    if (use_graph && (rc = ensure_graph(ctx, g, (int)(parity & 1))) != NNLBM_OK) return rc;
     for (int64_t k = 0; k < n;) {
         const int p = (int)((parity + k) & 1);
         if (use_graph && n - k >= kChainSteps) {
