@@ -813,12 +813,14 @@ int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
         }
     };
     std::vector<std::thread> team;
-    try {
-        team.reserve(threads);
-        for (size_t t = 0; t < threads; ++t) team.emplace_back(work);
-    } catch (...) {
-        // fewer threads, or none: then this thread converts
-    }
+    auto start_team = [&] {
+        try {
+            team.reserve(threads);
+            for (size_t t = 0; t < threads; ++t) team.emplace_back(work);
+        } catch (...) {
+            // fewer threads, or none: then this thread converts
+        }
+    };
     // chunk k is copied once its slot is empty, as far ahead as there are slots
     cudaError_t e = cudaSuccess;
     size_t issued = 0;
@@ -837,6 +839,8 @@ int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
         }
         if (e == cudaSuccess) e = cudaEventSynchronize(ctx->read_done[k % kReadSlots]);
         if (e != cudaSuccess) break;
+        // only now, so that the threads do not spin while queued steps run
+        if (k == 0) start_team();
         ready.store(k + 1, std::memory_order_release);
         if (team.empty()) convert(k);
     }

@@ -6,11 +6,13 @@ in two threads.
 from __future__ import annotations
 
 import threading
+import time
 
 import numpy as np
 import pytest
 
 from nonnewlbm_b200 import CaseSpec, Lattice, capi
+from nonnewlbm_b200 import geometry as G
 
 pytestmark = pytest.mark.gpu
 SMALL, LARGE = (97, 89, 83), (163, 167, 171)   # a single-precision field: 2.9 MB, 18.6 MB
@@ -62,3 +64,19 @@ def test_two_contexts_in_two_threads():
     for lat in lats:
         lat.close()
     assert not bad
+
+
+def test_converting_threads_start_with_the_first_data():
+    """A large field is asked for while steps are queued: nothing but the calling thread's own wait
+    takes processor time until they have run (five threads convert this field)."""
+    with Lattice(CaseSpec(LARGE, collision="CUM", dtype="f64")) as lat:
+        lat.set_map(np.full(LARGE[::-1], G.MAP_PERIODIC, dtype=np.uint8))
+        lat.init_equilibrium()
+        lat.step(2, macro=True)
+        lat.macro(0)
+        lat.step(1500, macro=True, wait=False)
+        wall, cpu = time.perf_counter(), time.process_time()
+        lat.macro(0)
+        wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+        assert wall > 0.2              # the steps were still queued
+        assert cpu <= 2.0 * wall
