@@ -1281,7 +1281,7 @@ int nnlbm_set_map(nnlbm_ctx* ctx, int ic, const uint8_t* map)
                 const unsigned xface = (x0 == 0 ? 1u : 0u) | (nx - 1 - x0 < kChunk ? 1u << (nx - 1 - x0) : 0u);
                 const bool plain = !face && !(ch.fluid & xface) && !(ch.cflags & CH_HW);
                 // nodes of x planes that are lanes of a plain chunk leave with the row's own stores
-                // (a node has one inward cell; of two cells that would serve one lane, neither does)
+                // (a node has one inward cell, so it is in one of the two masks)
                 const unsigned self = ~ch.fluid;
                 if (plain && hw.empty()) {
                     cn.row_l = (cn.xneg >> 1) & self;

@@ -443,7 +443,7 @@ __device__ __noinline__ void stored_equilibrium(int eq, typename Storage<DT>::CT
 // the open-plane nodes among the lanes of a chunk (CH_ROW), called by the whole warp between the
 // collision and the stores: rho, u are each lane's pre-collision values, f the values it stores.
 // Returns whether this lane is such a node, with f its equilibrium
-template <int DT, bool ODD>
+template <int DT>
 __device__ __forceinline__ bool row_nodes(const CaseArgs<typename Storage<DT>::CT>& a, const NodeWords& nw, int lane, int c, int step,
                                           int flags, typename Storage<DT>::CT rho, typename Storage<DT>::CT ux,
                                           typename Storage<DT>::CT uy, typename Storage<DT>::CT uz, typename Storage<DT>::CT* f)
@@ -634,21 +634,23 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 
 // register budget per thread of each step-kernel variant.  FP64 arithmetic may use all 255; the
 // paired form (two cells per thread) gets NNLBM_PAIR_REGS (two 256-thread blocks per SM).  The
-// one-cell forms run in 64-thread blocks, so that the budget sets the warps per SM almost
-// continuously, and a few spilled values cost less than the warps that hide the loads; us a step
-// by budget, one B200:
+// one-cell forms run in blocks of 256 threads, or of 64 or 128 where autotuning finds them faster; small
+// blocks let the budget set the warps per SM almost continuously.  A few spilled values cost less
+// than the warps that hide the loads.  us a step by budget, all on this code in one run, one B200
+// (boxes, junction and batch autotuned, KBC in 256-thread blocks):
 //   FP32 storage, NNLBM_CHUNK_REGS_F32       72     80     88     96
-//     cumulant, box 192x144x120             153    157    172    174
-//     with mean/rms sums                    195    193    196    205
-//     junction (CY, sums)                  30.3   29.5
-//     eight junctions                      63.8   61.2
+//     cumulant, box 192x144x120           152.7  159.4  169.0  167.1
+//     with mean/rms sums                  195.7  194.9  196.7  195.3
+//     junction (CY, sums)                  27.5   27.4   27.7   27.1
+//     eight junctions                      63.8   61.4   65.1   63.5
 //   16-bit cumulant, NNLBM_CHUNK_REGS_CUM16  64     72     80     88
-//     box 384x288x240, FP16                 842    849    999   1080
-//   KBC, NNLBM_KBC_REGS                      72     80     96    104    128
-//     KBC_N4, FP32 box 176x144x112          206    189    211    209    196
-//     KBC_N4 FP16 junction x0.75           17.8   17.6   19.4   19.0   18.4
-// 16-bit BGK and MRT_LES keep NNLBM_CHUNK_REGS: autotuned, 180.9 to 181.9 us at 64 to 96 on the box
-// of 211x163x137
+//     box 384x288x240, FP16                 928   1049    981   1083
+//   16-bit BGK and MRT_LES, NNLBM_CHUNK_REGS 64     72     80
+//     BGK, box 211x163x137, BF16          190.5  192.7  212.5
+//   KBC, FP32 storage, NNLBM_KBC_REGS        72     80     96    112    128
+//     KBC_N4, box 176x144x112             204.9  196.5  210.3  201.1  198.0
+//   KBC, 16-bit storage, NNLBM_KBC_REGS16    64     72     80     96    112    128
+//     KBC_N4, junction x0.75, FP16         51.8   28.1   25.9   22.9   23.2   22.1
 #ifndef NNLBM_PAIR_REGS
 #define NNLBM_PAIR_REGS 128
 #endif
@@ -665,7 +667,7 @@ __host__ __device__ constexpr bool pairs_chunks(int dt, int col)
 #define NNLBM_CHUNK_REGS_F32 80
 #endif
 #ifndef NNLBM_CHUNK_REGS_CUM16
-#define NNLBM_CHUNK_REGS_CUM16 72
+#define NNLBM_CHUNK_REGS_CUM16 64
 #endif
 template <int DT, int COL, bool PAIR>
 struct StepRegs {
@@ -816,7 +818,7 @@ __device__ __forceinline__ void fluid_chunk(const CaseArgs<typename Storage<DT>:
     // face wraps around the row
     int cm = c, cp = c;
     if (ch.cflags & CH_ROW) {
-        if (row_nodes<DT, ODD>(a, nw, lane, c, step, flags, rho, ux, uy, uz, f)) {
+        if (row_nodes<DT>(a, nw, lane, c, step, flags, rho, ux, uy, uz, f)) {
             put = true;
             if (ODD) {
                 const int x = c % a.nx;
