@@ -509,6 +509,7 @@ int upload_group(nnlbm_ctx* ctx, Group& g)
     ga.n_chunks = g.n_chunks;
     ga.gather = g.d_gather;
     ga.n_gather = g.n_gather;
+    ga.wait_first = g.n_gather == 0 || g.any_refd;
     ga.nodes = g.d_nodes;
     ga.n_nodes = g.n_nodes;
     ga.bc_prof = (const CT*)g.d_bc_prof;
@@ -546,19 +547,21 @@ bool can_stage(const nnlbm_ctx* ctx, const Group& g)
 }
 
 // the kernels of one step with the group arguments `args` (no host synchronisation); `odd` is
-// the A-A parity.  `chained`: each kernel but the gather as a programmatic dependent of the one
-// before it; `only_step`: without the kernels before the step kernel itself
+// the A-A parity.  `chained`: each kernel as a programmatic dependent of the one before it, but a gather
+// directly before the step kernel; `only_step`: without the kernels before the step kernel itself
 int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool odd, bool chained, bool only_step = false)
 {
     const AuxLaunchers& A = aux_launchers(g.dtype);
     const int per_block = g.block / kChunk;
     auto blocks = [](int warps, int per) { return dim3(std::max((warps + per - 1) / per, 1)); };
+    // directly before the step kernel the gather is not chained (pdl_wait)
+    if (!only_step && g.n_gather > 0)
+        A.gather(odd, chained && g.any_refd, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     if (!only_step && g.any_refd) {
         const dim3 rgrid = blocks(g.n_chunks, per_block); // one warp per chunk
         A.refd_velocity(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
         A.refd_stress(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
     }
-    if (!only_step && g.n_gather > 0) A.gather(odd, false, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     dim3 grid = blocks(step_warps(g), per_block), block(g.block);
     int form = g.paired ? FORM_PAIRED : FORM_ONE;
     if (g.staged) {

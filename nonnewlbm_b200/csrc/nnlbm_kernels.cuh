@@ -189,7 +189,8 @@ struct GroupArgs {
     const CaseArgs<CT>* cases;
     const Chunk* chunks;
     const ChunkNodes* chunk_nodes;  // of the serving chunks
-    int n_chunks, pad0;
+    // wait_first: the kernel before the step kernel is not the gather, which it may overtake
+    int n_chunks, wait_first;
     const int4* gather;        // {cell, case, node index, label} of the open-plane nodes
     int n_gather, n_nodes;
     const int4* nodes;         // [n_nodes] {cell, case, node index} of the boundary nodes with a lane of their own
@@ -224,16 +225,20 @@ __host__ __device__ constexpr int args_mode(int n_cases)
 // Programmatic dependent launch: the kernels of a step, and the steps of a call, are chained, so
 // that the launch of each overlaps the end of the one before.  A step launches the open-plane
 // gather, where it has nodes to gather, and the step kernel; with the finite-difference
-// Carreau-Yasuda coupling its velocity and strain kernels first, each waiting for the one before.
+// Carreau-Yasuda coupling its velocity and strain kernels between the two.
 //   - A chained kernel waits for the one before ahead of everything that a step changes; only work-list
 //     records, wall masks and labels are read earlier.
-//   - The gather is not chained: it starts once the kernel before it has ended, and lets the step kernel
-//     start at once, which so sees all that the kernels before the gather wrote without a wait of its
-//     own (a wait in the gather alone would order nothing for the step kernel).  The slots that
-//     the gather reads are overwritten by the step: the chunks that hold them (CH_WAIT) and the node
-//     warps wait for it before their first store.  us a step, gather chained -> not: FP32 box
-//     192x144x120 158.9 -> 153.0, KBC_N4 box 192.3 -> 185.2, ref-fd junction x0.5 28.7 -> 29.0; with a
-//     step kernel that waits for the gather first 162.9, 197.4, 32.5.
+//   - Directly before the step kernel the gather is not chained: it starts once the kernel before it
+//     has ended, and lets the step kernel start at once, which so sees all that the kernels before the
+//     gather wrote without a wait of its own (a wait in the gather alone would order nothing for the
+//     step kernel).  The slots that the gather reads are overwritten by the step: the chunks that hold
+//     them (CH_WAIT) and the node warps wait for it before their first store.  us a step, gather
+//     chained -> not: FP32 box 192x144x120 158.9 -> 153.0, KBC_N4 box 192.3 -> 185.2; with a step
+//     kernel that waits for the gather first 162.9, 197.4.
+//   - With the finite-difference coupling the gather, which reads populations only, is the first
+//     kernel of a step, and it and the three after it are chained and wait for the one before: 1000
+//     steps of a junction x0.5 and its fields take 35.9 ms, with an unchained gather behind the
+//     strain kernel 37.6.
 //   - The step kernel itself leaves the next kernel's start to its own end: with an earlier trigger
 //     the next step's blocks come up while this one's are running, and measured slower (pipe
 //     96x32x32 7.5 us a step against 6.5, junction 31.2 against 30.1).
@@ -1177,7 +1182,7 @@ __global__ void __launch_bounds__(256) __maxnreg__((StepRegs<DT, COL, PAIR>::val
         if (w < g.n_chunks) ch = g.chunks[w];
         if (early) hwm = chunk_walls<ODD>(case_args<ARGS>(g, ch.cflags & CH_CASE_MASK), ch, lane);
     }
-    if (g.n_gather == 0) pdl_wait();
+    if (g.wait_first) pdl_wait();
     const int step = g.cursor[ODD ? 1 : 0];
     if (blockIdx.x == 0 && threadIdx.x == 0) g.cursor[ODD ? 0 : 1] = step + 1;
     // the step's flags are the same for every case of the group.  They are read ahead of the
@@ -1406,7 +1411,7 @@ __global__ void __launch_bounds__(kStagedThreads) __maxnreg__((StepRegs<DT, COL,
     // otherwise hold
     __shared__ int loop_state[G::warps][2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (g.n_gather == 0) pdl_wait();
+    if (g.wait_first) pdl_wait();
     const int step = g.cursor[ODD ? 1 : 0];
     if (blockIdx.x == 0 && threadIdx.x == 0) g.cursor[ODD ? 0 : 1] = step + 1;
     const int flags = case_args<ARGS>(g, 0).ctl[step].flags;
@@ -1539,6 +1544,7 @@ __global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupA
 {
     using CT = typename Storage<DT>::CT;
     pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.n_gather) return;
     // {cell, case, node index, label}: the stencil loads depend on nothing but this record
