@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -815,15 +816,32 @@ int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
             convert(k);
         }
     };
-    std::vector<std::thread> team;
-    auto start_team = [&] {
-        try {
-            team.reserve(threads);
-            for (size_t t = 0; t < threads; ++t) team.emplace_back(work);
-        } catch (...) {
-            // fewer threads, or none: then this thread converts
+    // the threads are made while queued steps run and sleep until the first buffer's copy is there: made
+    // only then, they cost 40 MB of output fields behind 300 steps 0.2 of 8.5 ms
+    std::mutex gate;
+    std::condition_variable opened;
+    bool open = false;
+    auto open_gate = [&] {
+        {
+            std::lock_guard<std::mutex> l(gate);
+            open = true;
         }
+        opened.notify_all();
     };
+    std::vector<std::thread> team;
+    try {
+        team.reserve(threads);
+        for (size_t t = 0; t < threads; ++t)
+            team.emplace_back([&] {
+                {
+                    std::unique_lock<std::mutex> l(gate);
+                    opened.wait(l, [&] { return open; });
+                }
+                work();
+            });
+    } catch (...) {
+        // fewer threads, or none: then this thread converts
+    }
     // chunk k is copied once its slot is empty, as far ahead as there are slots
     cudaError_t e = cudaSuccess;
     size_t issued = 0;
@@ -842,13 +860,16 @@ int read_array(nnlbm_ctx* ctx, const S* src, D* out, size_t n)
         }
         if (e == cudaSuccess) e = cudaEventSynchronize(ctx->read_done[k % kReadSlots]);
         if (e != cudaSuccess) break;
-        // only now, so that the threads do not spin while queued steps run
-        if (k == 0) start_team();
         ready.store(k + 1, std::memory_order_release);
+        if (k == 0 && !team.empty()) open_gate();
         if (team.empty()) convert(k);
     }
-    if (e != cudaSuccess) failed.store(true);
-    else if (!team.empty()) work();
+    if (e != cudaSuccess) {
+        failed.store(true);
+        open_gate();
+    } else if (!team.empty()) {
+        work();
+    }
     for (std::thread& t : team) t.join();
     if (e != cudaSuccess) {
         cudaStreamSynchronize(ctx->stream); // no copy still writes the buffers
