@@ -294,7 +294,8 @@ int nnlbm_step_info(nnlbm_ctx* ctx, int ic, int64_t* fluid_cells, int64_t* bc_ce
 /* Run n_steps of case ic as individual launches with CUDA events around every kernel and
  * return the summed device milliseconds per kernel kind in ms[5] = {open-plane gather,
  * fused step, open-plane write, CY_REF_FD velocity, CY_REF_FD strain} and the launch counts
- * in launches[5].  The steps are real steps (the lattice advances).  No reference
+ * in launches[5]; with CY_REF_FD the velocity kernel gathers too, and no gather is launched.
+ * The steps are real steps (the lattice advances).  No reference
  * counterpart (the reference logs wall-clock MLUPS, core.h:1440-1469). */
 int nnlbm_profile_step(nnlbm_ctx* ctx, int ic, int64_t n_steps, int flags, double* ms, int64_t* launches);
 

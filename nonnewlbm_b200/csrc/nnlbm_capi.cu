@@ -548,20 +548,20 @@ bool can_stage(const nnlbm_ctx* ctx, const Group& g)
 }
 
 // the kernels of one step with the group arguments `args` (no host synchronisation); `odd` is
-// the A-A parity.  `chained`: each kernel as a programmatic dependent of the one before it, but a gather
-// directly before the step kernel; `only_step`: without the kernels before the step kernel itself
+// the A-A parity.  `chained`: each kernel but the gather as a programmatic dependent of the one
+// before it; `only_step`: without the kernels before the step kernel itself
 int launch_step_kernels(nnlbm_ctx* ctx, const Group& g, const void* args, bool odd, bool chained, bool only_step = false)
 {
     const AuxLaunchers& A = aux_launchers(g.dtype);
     const int per_block = g.block / kChunk;
     auto blocks = [](int warps, int per) { return dim3(std::max((warps + per - 1) / per, 1)); };
-    // directly before the step kernel the gather is not chained (pdl_wait)
-    if (!only_step && g.n_gather > 0)
-        A.gather(odd, chained && g.any_refd, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     if (!only_step && g.any_refd) {
-        const dim3 rgrid = blocks(g.n_chunks, per_block); // one warp per chunk
-        A.refd_velocity(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
-        A.refd_stress(odd, chained, rgrid, dim3(g.block), ctx->stream, args);
+        // one warp per chunk, and the velocity kernel's for 32 gathered nodes each
+        A.refd_velocity(odd, chained, blocks(g.n_chunks + (g.n_gather + 31) / 32, per_block), dim3(g.block), ctx->stream, args);
+        A.refd_stress(odd, chained, blocks(g.n_chunks, per_block), dim3(g.block), ctx->stream, args);
+    } else if (!only_step && g.n_gather > 0) {
+        // not chained (pdl_wait)
+        A.gather(odd, false, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, args);
     }
     dim3 grid = blocks(step_warps(g), per_block), block(g.block);
     int form = g.paired ? FORM_PAIRED : FORM_ONE;
@@ -1917,7 +1917,7 @@ int nnlbm_step_info(nnlbm_ctx* ctx, int ic, int64_t* fluid_cells, int64_t* bc_ce
     if ((rc = prepare_group(ctx, g)) != NNLBM_OK) return rc;
     if (fluid_cells) *fluid_cells = c.n_fluid;
     if (bc_cells) *bc_cells = c.n_bc;
-    if (launches_per_step) *launches_per_step = 1 + (g.n_gather > 0 ? 1 : 0) + (g.any_refd ? 2 : 0);
+    if (launches_per_step) *launches_per_step = 1 + (g.any_refd ? 2 : g.n_gather > 0 ? 1 : 0);
     if (bytes_per_step) *bytes_per_step = (double)c.n_fluid * (54.0 * kStorageBytes[c.d.dtype] + 1.0);
     return NNLBM_OK;
 }
@@ -1933,7 +1933,9 @@ int nnlbm_profile_step(nnlbm_ctx* ctx, int ic, int64_t n_steps, int flags, doubl
     const AuxLaunchers& A = aux_launchers(g.dtype);
     const int per_block = g.block / kChunk;
     const dim3 cblk(g.block);
-    const dim3 rgrid((std::max(g.n_chunks, 1) + per_block - 1) / per_block); // one warp per chunk
+    // one warp per chunk, and the velocity kernel's for 32 gathered nodes each
+    const dim3 rgrid((std::max(g.n_chunks, 1) + per_block - 1) / per_block);
+    const dim3 vgrid((std::max(g.n_chunks + (g.n_gather + 31) / 32, 1) + per_block - 1) / per_block);
     for (int i = 0; i < 5; ++i) { ms[i] = 0; launches[i] = 0; }
     const int64_t parity = ctx->cases[g.cases[0]].parity;
     // kinds: 0 gather, 1 step, 3 CY_REF_FD velocity, 4 CY_REF_FD strain
@@ -1950,12 +1952,12 @@ int nnlbm_profile_step(nnlbm_ctx* ctx, int ic, int64_t n_steps, int flags, doubl
         const bool odd = ((parity + k) & 1) != 0;
         if (mark(-1)) return set_err(ctx, NNLBM_ERR_CUDA, "event record failed");
         if (g.any_refd) {
-            A.refd_velocity(odd, false, rgrid, cblk, ctx->stream, g.args.data());
+            A.refd_velocity(odd, false, vgrid, cblk, ctx->stream, g.args.data());
             mark(3);
             A.refd_stress(odd, false, rgrid, cblk, ctx->stream, g.args.data());
             mark(4);
         }
-        if (g.n_gather > 0) {
+        if (g.n_gather > 0 && !g.any_refd) {
             A.gather(odd, false, dim3((g.n_gather + 63) / 64), dim3(64), ctx->stream, g.args.data());
             mark(0);
         }

@@ -225,20 +225,19 @@ __host__ __device__ constexpr int args_mode(int n_cases)
 // Programmatic dependent launch: the kernels of a step, and the steps of a call, are chained, so
 // that the launch of each overlaps the end of the one before.  A step launches the open-plane
 // gather, where it has nodes to gather, and the step kernel; with the finite-difference
-// Carreau-Yasuda coupling its velocity and strain kernels between the two.
+// Carreau-Yasuda coupling its velocity kernel, which gathers too, and its strain kernel first.
 //   - A chained kernel waits for the one before ahead of everything that a step changes; only work-list
 //     records, wall masks and labels are read earlier.
-//   - Directly before the step kernel the gather is not chained: it starts once the kernel before it
-//     has ended, and lets the step kernel start at once, which so sees all that the kernels before the
+//   - The gather is not chained: it starts once the kernel before it has ended, and lets the step kernel start at once, which so sees all that the kernels before the
 //     gather wrote without a wait of its own (a wait in the gather alone would order nothing for the
 //     step kernel).  The slots that the gather reads are overwritten by the step: the chunks that hold
 //     them (CH_WAIT) and the node warps wait for it before their first store.  us a step, gather
 //     chained -> not: FP32 box 192x144x120 158.9 -> 153.0, KBC_N4 box 192.3 -> 185.2; with a step
 //     kernel that waits for the gather first 162.9, 197.4.
-//   - With the finite-difference coupling the gather, which reads populations only, is the first
-//     kernel of a step, and it and the three after it are chained and wait for the one before: 1000
-//     steps of a junction x0.5 and its fields take 35.9 ms, with an unchained gather behind the
-//     strain kernel 37.6.
+//   - With the finite-difference coupling all three kernels are chained and wait for the one before
+//     (wait_first).  us a step of a junction x0.5, by where its nodes are gathered: an unchained kernel
+//     behind the strain kernel 32.3, a chained one ahead of the velocity kernel 31.7, the velocity
+//     kernel's own warps 28.7.
 //   - The step kernel itself leaves the next kernel's start to its own end: with an earlier trigger
 //     the next step's blocks come up while this one's are running, and measured slower (pipe
 //     96x32x32 7.5 us a step against 6.5, junction 31.2 against 30.1).
@@ -1540,12 +1539,9 @@ __device__ __forceinline__ void pull_triples(const CaseArgs<typename Storage<DT>
 }
 
 template <int DT, bool ODD, int ARGS>
-__global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupArgs<typename Storage<DT>::CT> g)
+__device__ __forceinline__ void gather_node(const GroupArgs<typename Storage<DT>::CT>& g, int t)
 {
     using CT = typename Storage<DT>::CT;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.n_gather) return;
     // {cell, case, node index, label}: the stencil loads depend on nothing but this record
     // (and the case's arguments, from the parameters where the group is small)
@@ -1590,6 +1586,13 @@ __global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupA
     g.bc_buf[4 * k] = rho; g.bc_buf[4 * k + 1] = ux; g.bc_buf[4 * k + 2] = uy; g.bc_buf[4 * k + 3] = uz;
 }
 
+template <int DT, bool ODD, int ARGS>
+__global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupArgs<typename Storage<DT>::CT> g)
+{
+    pdl_launch_dependents();
+    gather_node<DT, ODD, ARGS>(g, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // ---------------------------------------------------------------------------------------
 // NNLBM_CY_REF_FD phases 1 and 2 (core.h:1176-1258): velocity of the post-streaming state
 // of every FLUID cell with the force of the previous step, then the finite-difference
@@ -1600,15 +1603,21 @@ __global__ void __launch_bounds__(64) k_bc_gather(const __grid_constant__ GroupA
 // labels) is read before the wait.  A FLUID cell lies off every face, so its pull is the step's own:
 // slot q at the cell (even) or slot opp(q) at x - c_q (odd), a population that a wall reflects
 // from slot q at the cell in both; the slot bases of the step give all 27 addresses.  A step of a
-// junction x0.5 (FP32, four kernels): 31.3 -> 28.7 us against clamped and wrapped coordinates for
-// every population and launches that waited for one another's end.
+// junction x0.5 (FP32, with an unchained gather of its own): 31.3 -> 28.7 us against clamped and wrapped
+// coordinates for every population and launches that waited for one another's end.
+// The first warps of the velocity kernel gather the open-plane nodes, which reads populations only.
 template <int DT, bool ODD, int ARGS>
 __global__ void __launch_bounds__(256) k_refd_velocity(const __grid_constant__ GroupArgs<typename Storage<DT>::CT> g)
 {
     using S = Storage<DT>;
     using CT = typename S::CT;
     const int lane = threadIdx.x & 31;
-    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) - ((g.n_gather + 31) >> 5);
+    if (warp < 0) {
+        pdl_wait();
+        gather_node<DT, ODD, ARGS>(g, blockIdx.x * blockDim.x + threadIdx.x);
+        return;
+    }
     Chunk ch{};
     if (warp < g.n_chunks) ch = g.chunks[warp];
     const CaseArgs<CT>& a = case_args<ARGS>(g, ch.cflags & CH_CASE_MASK);
