@@ -231,8 +231,7 @@ __device__ __forceinline__ f2 cy_nu_from_central(f2 Pxx, f2 Pyy, f2 Pzz, f2 Cxy,
 // for FP32 (DT = 1), f_q for FP64 (DT = 0).  (Those of the 16-bit types: nnlbm_physics16.cuh.)
 // Every moment is linear in them, so the weights meet a handful of moments (or the factors of
 // the equilibrium) instead of each of the 27 populations on the way in and out, and a moment
-// of g carries no rounding of the rest state.  Against populations shifted and scaled one by one, with the
-// moments summed per use, this halves the instructions of a step.
+// of g carries no rounding of the rest state.
 //
 // PLANES (one cell in single precision): the planes x = -1 and x = 0 run as f2 pairs on the
 // packed FP32 pipe, the plane x = +1 scalar.
@@ -386,7 +385,8 @@ __device__ __forceinline__ void to_pops(V& a, V& b, V& c)
     c = p;
 }
 
-// scaled central moments of a cell after the collision: the halves and quarters of the second order (x = s200/2, a = s110/4, ...) and the density
+// scaled central moments of a cell after the collision: the halves and quarters of the second
+// order (x = s200/2, a = s110/4, ...) and the density
 template <class CT>
 struct CumPost { CT r, x, y, z, a, b, c; };  // a: 110, b: 101, c: 011
 
