@@ -27,10 +27,10 @@
 // stencil re-centred one cell inward (sim_tcpc.cu:242-273, lbm_bc.h:147-152).  Where that
 // inward cell collides and lies off every face, the stencil is the cell's own pull, so the
 // cell's thread writes the node's equilibrium into the node's slots (serve_nodes).  For the
-// other nodes k_bc_gather computes density / velocity from the pre-step state before the
-// step kernel runs, and the node warps of the step kernel write each node's equilibrium
-// into the node's own slots, which no other cell touches within the step.  GEO_INFLOW
-// nodes take their prescribed velocity and need no gather.
+// other nodes k_bc_gather (k_refd_velocity, where there is one) computes density / velocity from
+// the pre-step state before the step kernel runs, and the node warps of the step kernel write
+// each node's equilibrium into the node's own slots, which no other cell touches within the
+// step.  GEO_INFLOW nodes take their prescribed velocity and need no gather.
 #pragma once
 
 #include <cuda.h>
